@@ -40,6 +40,11 @@ static const int kNDep = 5;
 static const int kPassCand[][2] = {{ORBIT_PASS_THREADS, 2048}, {ORBIT_PASS_THREADS, 4096}, {ORBIT_PASS_THREADS, 8192},
                                    {ORBIT_PASS_THREADS, 16384}};
 static const int kNPass = 4;
+// After the fixed shapes: particles per block such that the class's blocks
+// make one wave (one block per SM), or two.  A block's prologue (its copy of
+// the potential, the constants) is then paid once or twice per SM.
+static const int kNWave = 2;
+static const int kMaxDep = kNDep + kNWave, kMaxPass = kNPass + kNWave;
 
 struct BatchClass {
   int nx = 0, ny = 0, nz = 0;
@@ -53,6 +58,7 @@ struct BatchClass {
   PassJob* d_pass = nullptr;       // (nsc + 1) tables of mem.size() jobs: [0] no kick, [1 + i] kick i
   std::vector<BlockMap> dep_maps;  // one per deposit candidate
   std::vector<BlockMap> pass_maps; // one per pass candidate
+  int dep_cand[kMaxDep][2] = {}, pass_cand[kMaxPass][2] = {};  // {threads, particles per block}
   int dep_sel = 0, pass_sel = 0;
   std::string dep_tag, pass_tag;   // profile names of the class's deposit and kick passes
   cudaStream_t st = nullptr;
@@ -63,6 +69,7 @@ struct BatchClass {
 struct Tuner {
   struct Rec {
     int cls, stage, cand;  // stage 0 deposit, 1 pass
+    float weight;          // the launch's work per particle, relative
     cudaEvent_t a, b;
   };
   std::vector<Rec> recs;
@@ -130,6 +137,31 @@ static void free_graphs(orbit_batch_t* bt) {
 static bool sync_same(const orbit_sync_t& a, const orbit_sync_t& b) {
   return a.beta == b.beta && a.gamma == b.gamma && a.momentum == b.momentum && a.charge == b.charge &&
          a.classical_radius == b.classical_radius && a.macrosize == b.macrosize && a.mass == b.mass;
+}
+
+// The smallest number of particles per block with which the class's members
+// take at most `waves` blocks per SM.
+static int wave_chunk(const orbit_batch_t* bt, const BatchClass& c, int waves, int per) {
+  long long total = 0;
+  int nmax = 1;
+  for (int m : c.mem) {
+    total += bt->bunches[m]->n;
+    nmax = std::max(nmax, bt->bunches[m]->n);
+  }
+  const int cap = waves * num_sms() / per;
+  auto blocks = [&](int chunk) {
+    long long nb = 0;
+    for (int m : c.mem) nb += std::max(1, (bt->bunches[m]->n + chunk - 1) / chunk);
+    return nb;
+  };
+  int lo = (int)std::max(256ll, total / std::max(1, cap)), hi = nmax;
+  if (lo >= hi || blocks(hi) > cap) return std::max(lo, hi);
+  while (lo < hi) {
+    const int mid = lo + (hi - lo) / 2;
+    if (blocks(mid) <= cap) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
 }
 
 // Blocks of each member for `chunk` particles per `per` blocks.
@@ -215,17 +247,26 @@ static int build_tables(orbit_batch_t* bt, BatchClass& c) {
       P.status = b->d_status;
       P.sa = sa;
       P.knl = p->d_knl;
+      P.prep = k->d_prep;
     }
   }
   int rc = upload(&c.d_solve, sj);
   if (!rc) rc = upload(&c.d_dep, dj);
   if (!rc) rc = upload(&c.d_pass, pj);
   if (rc) return rc;
-  c.dep_maps.resize(kNDep);
-  c.pass_maps.resize(kNPass);
+  c.dep_maps.resize(kMaxDep);
+  c.pass_maps.resize(kMaxPass);
   const int bands = batch_deposit_bands(c.proto);
-  for (int q = 0; q < kNDep && !rc; ++q) rc = build_map(bt, c, kDepCand[q][1], bands, c.dep_maps[q]);
-  for (int q = 0; q < kNPass && !rc; ++q) rc = build_map(bt, c, kPassCand[q][1], 1, c.pass_maps[q]);
+  for (int q = 0; q < kMaxDep && !rc; ++q) {
+    c.dep_cand[q][0] = q < kNDep ? kDepCand[q][0] : kDepCand[0][0];
+    c.dep_cand[q][1] = q < kNDep ? kDepCand[q][1] : wave_chunk(bt, c, 1 + q - kNDep, bands);
+    rc = build_map(bt, c, c.dep_cand[q][1], bands, c.dep_maps[q]);
+  }
+  for (int q = 0; q < kMaxPass && !rc; ++q) {
+    c.pass_cand[q][0] = ORBIT_PASS_THREADS;
+    c.pass_cand[q][1] = q < kNPass ? kPassCand[q][1] : wave_chunk(bt, c, 1 + q - kNPass, 1);
+    rc = build_map(bt, c, c.pass_cand[q][1], 1, c.pass_maps[q]);
+  }
   return rc;
 }
 
@@ -292,11 +333,12 @@ static bool key_same(const orbit_batch_t* bt) {
   return true;
 }
 
-static int rec_begin(Tuner* tu, int cls, int stage, int cand, cudaStream_t s, Tuner::Rec* r) {
+static int rec_begin(Tuner* tu, int cls, int stage, int cand, float weight, cudaStream_t s, Tuner::Rec* r) {
   if (!tu) return ORBIT_OK;
   r->cls = cls;
   r->stage = stage;
   r->cand = cand;
+  r->weight = weight;
   ORBIT_CUDA(cudaEventCreate(&r->a));
   ORBIT_CUDA(cudaEventCreate(&r->b));
   ORBIT_CUDA(cudaEventRecord(r->a, s));
@@ -325,41 +367,43 @@ static int enqueue_class_turn(orbit_batch_t* bt, int ci, cudaStream_t s, bool pr
     return km;
   };
   // (only kick passes are timed: the prologue pass has no kick)
-  auto pass = [&](int table, const Seg& sg, bool kick, bool ext, int cand) -> int {
+  auto pass = [&](int table, const Seg& sg, bool kick, bool ext, int cand, int km) -> int {
     Tuner* t = kick ? tu : nullptr;
     Tuner::Rec r{};
-    int rc = rec_begin(t, ci, 1, cand, s, &r);
+    int rc = rec_begin(t, ci, 1, cand, (float)(6 + sg.b - sg.a), s, &r);
     if (rc) return rc;
-    rc = batch_enqueue_pass(c.d_pass + (size_t)table * nm, c.pass_maps[cand], kPassCand[cand][0], kick ? 1 : 0, ext,
-                            kick && c.ksmem, c.kick_smem, sg.a, sg.b, km_of(sg), s, c.pass_tag.c_str());
+    rc = batch_enqueue_pass(c.d_pass + (size_t)table * nm, c.pass_maps[cand], c.pass_cand[cand][0], kick ? 1 : 0, ext,
+                            kick && c.ksmem, c.kick_smem, sg.a, sg.b, km, fixed_pass(sg, kick, km), s,
+                            c.pass_tag.c_str());
     if (rc) return rc;
     ++*nl;
     return rec_end(t, s, r);
   };
   int rc;
   if (prologue) {
-    rc = pass(0, plan.segs[0], false, true, c.pass_sel);
+    rc = pass(0, plan.segs[0], false, true, c.pass_sel, km_of(plan.segs[0]));
     if (rc) return rc;
   }
   for (int i = 0; i < nsc; ++i) {
     rc = batch_enqueue_green(c.d_solve, nm, c.proto, c.tune.fft_wide, s);
     if (rc) return rc;
     *nl += 3;
-    int dc = tu ? i % kNDep : c.dep_sel;
+    // (the shift by one each round keeps a candidate off the lattice's period)
+    int dc = tu ? (i + i / kMaxDep) % kMaxDep : c.dep_sel;
     Tuner::Rec r{};
-    rc = rec_begin(tu, ci, 0, dc, s, &r);
-    if (!rc) rc = batch_enqueue_deposit(c.d_dep, c.dep_maps[dc], c.proto, kDepCand[dc][0], s, c.dep_tag.c_str());
+    rc = rec_begin(tu, ci, 0, dc, 1.f, s, &r);
+    if (!rc) rc = batch_enqueue_deposit(c.d_dep, c.dep_maps[dc], c.proto, c.dep_cand[dc][0], s, c.dep_tag.c_str());
     if (!rc) rc = rec_end(tu, s, r);
     if (rc) return rc;
     ++*nl;
-    rc = batch_enqueue_solve(c.d_solve, nm, c.proto, c.tune.fft_wide, !c.ksmem, s);
+    const bool last = i == nsc - 1;
+    const Seg& sg = !last ? plan.segs[i + 1] : (wrap ? plan.wrap : plan.segs[nsc]);
+    const int km = km_of(sg);
+    rc = batch_enqueue_solve(c.d_solve, nm, c.proto, c.tune.fft_wide, !c.ksmem,
+                             fixed_pass(sg, true, km) ? c.d_pass + (size_t)(1 + i) * nm : nullptr, sg.a, sg.b, s);
     if (rc) return rc;
     *nl += c.ksmem ? 3 : 4;
-    int pc = tu ? i % kNPass : c.pass_sel;
-    bool last = i == nsc - 1;
-    if (!last) rc = pass(1 + i, plan.segs[i + 1], true, true, pc);
-    else if (wrap) rc = pass(1 + i, plan.wrap, true, true, pc);
-    else rc = pass(1 + i, plan.segs[nsc], true, false, pc);
+    rc = pass(1 + i, sg, true, !last || wrap, tu ? (i + i / kMaxPass) % kMaxPass : c.pass_sel, km);
     if (rc) return rc;
   }
   return ORBIT_OK;
@@ -451,6 +495,14 @@ static int probe_fft(orbit_batch_t* bt) {
   return rc;
 }
 
+// The chosen shapes as orbit_batch_class reports them.
+static void report_shapes(BatchClass& c) {
+  c.tune.dep_threads = c.dep_cand[c.dep_sel][0];
+  c.tune.dep_chunk = c.dep_cand[c.dep_sel][1];
+  c.tune.pass_threads = c.pass_cand[c.pass_sel][0];
+  c.tune.pass_chunk = c.pass_cand[c.pass_sel][1];
+}
+
 // Median time of each candidate shape over the tuning turn; the fastest
 // is kept.
 static int finish_tuning(orbit_batch_t* bt, Tuner& tu) {
@@ -459,12 +511,12 @@ static int finish_tuning(orbit_batch_t* bt, Tuner& tu) {
   for (auto& r : tu.recs) {
     float ms = 0.f;
     ORBIT_CUDA(cudaEventElapsedTime(&ms, r.a, r.b));
-    t[std::make_tuple(r.cls, r.stage, r.cand)].push_back(ms);
+    t[std::make_tuple(r.cls, r.stage, r.cand)].push_back(ms / r.weight);
   }
   for (size_t ci = 0; ci < bt->classes.size(); ++ci) {
     BatchClass& c = bt->classes[ci];
     for (int stage = 0; stage < 2; ++stage) {
-      int nc = stage == 0 ? kNDep : kNPass;
+      int nc = stage == 0 ? kMaxDep : kMaxPass;
       int best = 0;
       float bv = 1e30f;
       for (int q = 0; q < nc; ++q) {
@@ -478,10 +530,7 @@ static int finish_tuning(orbit_batch_t* bt, Tuner& tu) {
       if (stage == 0) c.dep_sel = best;
       else c.pass_sel = best;
     }
-    c.tune.dep_threads = kDepCand[c.dep_sel][0];
-    c.tune.dep_chunk = kDepCand[c.dep_sel][1];
-    c.tune.pass_threads = kPassCand[c.pass_sel][0];
-    c.tune.pass_chunk = kPassCand[c.pass_sel][1];
+    report_shapes(c);
   }
   bt->tuned = true;
   return ORBIT_OK;
@@ -732,10 +781,12 @@ int orbit_batch_set_tuning(orbit_batch_t* bt, int cls, const int* tuning) {
     return set_error(ORBIT_ERR_ARG, "orbit_batch_set_tuning: bad argument");
   BatchClass& c = bt->classes[cls];
   int ds = -1, ps = -1;
-  for (int q = 0; q < kNDep; ++q)
-    if (kDepCand[q][0] == tuning[0] && kDepCand[q][1] == tuning[1]) ds = q;
-  for (int q = 0; q < kNPass; ++q)
-    if (kPassCand[q][0] == tuning[2] && kPassCand[q][1] == tuning[3]) ps = q;
+  // the class's own shapes are known once it is compiled
+  auto is = [](const int cand[2], int threads, int chunk) { return cand[0] == threads && cand[1] == chunk; };
+  for (int q = kMaxDep - 1; q >= 0; --q)
+    if (is(q < kNDep ? kDepCand[q] : c.dep_cand[q], tuning[0], tuning[1])) ds = q;
+  for (int q = kMaxPass - 1; q >= 0; --q)
+    if (is(q < kNPass ? kPassCand[q] : c.pass_cand[q], tuning[2], tuning[3])) ps = q;
   if (ds < 0 || ps < 0 || (tuning[4] != 0 && tuning[4] != 1))
     return set_error(ORBIT_ERR_ARG, "orbit_batch_set_tuning: not one of the candidate shapes");
   if (bt->used) ORBIT_CUDA(cudaStreamSynchronize(bt->stream));

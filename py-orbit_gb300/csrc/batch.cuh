@@ -22,6 +22,7 @@ struct PassJob {
   unsigned* status;
   SetupArgs sa;
   double* knl;          // per-particle 1/(1+dp_p)
+  PassPrep* prep;       // the kick's and the fixed-point pass's constants
 };
 
 // One member's deposit (plain form).
@@ -76,8 +77,10 @@ int batch_enqueue_green(const SolveJob* jobs, int nm, const orbit_sc2p5d_t* prot
 // `tag` names the launch for orbit_batch_profile.
 int batch_enqueue_deposit(const DepJob* jobs, const BlockMap& bm, const orbit_sc2p5d_t* proto, int threads,
                           cudaStream_t s, const char* tag);
+// pass: the members' jobs of the fixed-point pass over maps [a, b) that
+// follows (its constants are made beside the forward rows), null for others.
 int batch_enqueue_solve(const SolveJob* jobs, int nm, const orbit_sc2p5d_t* proto, int fft_wide, bool phi_fix,
-                        cudaStream_t s);
+                        const PassJob* pass, int a, int b, cudaStream_t s);
 // The columns (forward, Green multiply, backward) and backward rows alone,
 // for timing the FFT schedules: they write only the work spectra, the
 // potentials and max |phi|, which the next solve and grid set-up replace.
@@ -92,9 +95,9 @@ int batch_deposit_bands(const orbit_sc2p5d_t* proto);
 
 // Batched fused pass (program.cu).  kf: 0 no kick, 1 plain kick; ksmem: the
 // kick keeps a fixed-point copy of the potential of `smem` bytes in shared
-// memory.
+// memory; fixed: the pass in fixed point (its own block size).
 int batch_enqueue_pass(const PassJob* jobs, const BlockMap& bm, int threads, int kf, bool ext, bool ksmem,
-                       size_t smem, int a, int b, int km, cudaStream_t s, const char* tag);
+                       size_t smem, int a, int b, int km, bool fixed, cudaStream_t s, const char* tag);
 // Largest pass-kick copy of the potential kept in shared memory.
 size_t batch_pass_smem_limit();
 

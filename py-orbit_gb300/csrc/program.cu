@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "sc2p5d.cuh"
+#include "passprep.cuh"
 #include "sc_device.cuh"
 #include "teapot.cuh"
 #include "batch.cuh"
@@ -27,6 +28,10 @@ static const int kPassSmem = 220 * 1024;
 // 65536 / ORBIT_PASS_THREADS.
 #ifndef ORBIT_PASS_THREADS
 #define ORBIT_PASS_THREADS 512
+#endif
+// The same of the fixed-point pass.
+#ifndef ORBIT_FX_THREADS
+#define ORBIT_FX_THREADS 640
 #endif
 
 // Copies n elements of global memory (written by an earlier kernel) into
@@ -65,8 +70,168 @@ __device__ __noinline__ void kick_consts_into(KickConst* k, KickFix* kf, const K
   if (kf) load_kick_fix(*kf, kick.st, k->fac, kick.nx, kick.ny, kick.nz);
 }
 
+// x 2^S to the nearest integer and back, by the conversion instructions (the
+// power of two joins the exponent): the FP64 pipe is otherwise idle in the
+// fixed-point pass.
+__device__ __forceinline__ long long cvt_to(double x, int S) {
+  return __double2ll_rn(__hiloint2double(__double2hiint(x) + (S << 20), __double2loint(x)));
+}
+__device__ __forceinline__ double cvt_from(long long v, int S) {
+  const double d = __ll2double_rn(v);
+  const int h = __double2hiint(d);
+  return __hiloint2double(h == 0 ? 0 : h - (S << 20), __double2loint(d));
+}
+
+// Cell and fraction (Q62) of tsc_fixed; false within a quarter cell of the
+// grid's edge or outside.
+__device__ __forceinline__ bool cell_fx(const FxGrid& g, long long x, int ncell, int& ic, long long& f) {
+  const long long t = fx::mul(g.a, fx::sp(x), g.c);
+  const int h = (int)(t >> 32);
+  const int i = (h + g.half) >> (g.F - 32);
+  ic = min(max(i, 1), ncell - 2);
+  f = (long long)((unsigned long long)t << (62 - g.F)) - ((long long)ic << 62);
+  return (h >= g.lo) & (h <= g.hi);
+}
+
+// The plain kick in fixed point; false: the particle takes the FP64 path.
+// Every particle lies in [zmin, zmax], the extent of the scan before it.
+__device__ __forceinline__ bool kick_fx(const FxPass& f, int nx, const long long* __restrict__ P,
+                                        const long long* __restrict__ Lm, fx::Part& t) {
+  int ix, iy;
+  long long gfx, gfy, gx, gy, lv;
+  const bool in = cell_fx(f.gx, t.x, nx, ix, gfx) & cell_fx(f.gy, t.y, f.ny, iy, gfy);
+  if (!in) return false;
+  if (f.nz > 1) {
+    const long long v = cvt_to(fma(t.z, f.az, f.cz), f.Fz);
+    const int i = min(max((int)(v >> f.Fz), 0), f.nz);
+    const long long w = (long long)((unsigned long long)(v - ((long long)i << f.Fz)) << (62 - f.Fz));
+    lv = fx::mul2(fx::sp((1ll << 62) - w), fx_of_pair(Lm[(i == 0 ? f.nz : i) - 1]), fx::sp(w),
+                  fx_of_pair(Lm[i == f.nz ? 0 : i]));
+  } else {
+    lv = fx::join(fx_of_pair(Lm[0])) >> 2;
+  }
+  grad_fixed(P, f.ny, ix, iy, gfx, gfy, gx, gy);
+  const fx::V l2 = fx::sp(lv << 2);
+  const long long px = fx::mul(fx::sp(gx << 4), l2), py = fx::mul(fx::sp(gy << 4), l2);
+  const long long dx = fx::mul(fx::sp(px << f.j), f.Cx), dy = fx::mul(fx::sp(py << f.j), f.Cy);
+  t.p += dx;
+  t.r += dy;
+  return fx::within(gx, (1 << 26) - 1) & fx::within(gy, (1 << 26) - 1) & fx::within(px, f.limj) &
+         fx::within(py, f.limj) & fx::within(dx, f.limk) & fx::within(dy, f.limk);
+}
+
+// What the FP64 routines of a fixed-point pass need, kept in shared memory,
+// with the extrema and magnitudes of the particles they take.
+struct FxFallback {
+  const KickConst* k;
+  const KickFix* kf;
+  const long long* P;
+  const long long* Lm;
+  double* c[5];
+  const double* dE;
+  const double* knl;
+  const KickArgs* kick;
+  const MapCtx* m;
+  const DevOp* ops;
+  int a, b;
+  unsigned long long mn[3], mx[3];
+  unsigned pm, sx, sp, n;
+  int bad;
+};
+
+// One particle by the FP64 routines: those the fixed-point form declines,
+// and all of a pass it cannot run.
+template <bool EXT>
+__device__ __noinline__ void pass_particle(FxFallback* f, int i, bool first) {
+  Part p;
+  p.x = f->c[0][i]; p.xp = f->c[1][i]; p.y = f->c[2][i]; p.yp = f->c[3][i]; p.z = f->c[4][i]; p.dE = f->dE[i];
+  p.knl = f->knl[i];
+  p.dp_p = dmul<ORBIT_SOFT_MUL & 1>(p.dE, f->m->dp_p_coeff);
+  p.knl_ok = true;
+  if (!f->k->skip && bnd_inside(f->kick->bnd, p.x, p.y)) {
+    if (!kick_fixed(*f->kf, f->P, f->Lm, p.x, p.y, p.z, p.xp, p.yp)) {
+      kick_plain(*f->k, f->kick->phi, f->kick->lam, p.x, p.y, p.z, p.xp, p.yp);
+    }
+  }
+  apply_ops<ORBIT_SOFT_MUL>(p, f->ops, f->a, f->b, *f->m);
+  if (EXT) {
+    ExtAcc e;
+    e.init();
+    e.add(p.x, p.y, p.z);
+    for (int c = 0; c < 3; ++c) {
+      atomicMin(&f->mn[c], e.mn[c]);
+      atomicMax(&f->mx[c], e.mx[c]);
+    }
+    if (e.bad) f->bad = 1;
+    MagAcc g;
+    g.init();
+    g.add(p.x, p.xp, p.y, p.yp, p.dE);
+    atomicMax(&f->pm, g.pm);
+    if (first) {
+      atomicAdd(&f->sx, g.sx);
+      atomicAdd(&f->sp, g.sp);
+      atomicAdd(&f->n, g.n);
+    }
+  }
+  f->c[0][i] = p.x; f->c[1][i] = p.xp; f->c[2][i] = p.y; f->c[3][i] = p.yp; f->c[4][i] = p.z;
+}
+
+// Extrema of a pass run in fixed point: x and y as integers (their
+// conversion to the stored doubles is monotonic), z as a key.
+struct ExtFx {
+  long long mn[2], mx[2];
+  unsigned long long zn, zx;
+  __device__ __forceinline__ void init() {
+    mn[0] = mn[1] = 0x7fffffffffffffffll;
+    mx[0] = mx[1] = -0x7fffffffffffffffll;
+    zn = ~0ull;
+    zx = 0ull;
+  }
+  __device__ __forceinline__ void add(long long x, long long y, double z) {
+    mn[0] = min(mn[0], x);
+    mx[0] = max(mx[0], x);
+    mn[1] = min(mn[1], y);
+    mx[1] = max(mx[1], y);
+    const unsigned long long k = dkey(z);
+    zn = min(zn, k);
+    zx = max(zx, k);
+  }
+  // As keys of the stored doubles.
+  __device__ __forceinline__ void join(ExtAcc& a, int S) const {
+    for (int c = 0; c < 2; ++c) {
+      if (mn[c] > mx[c]) continue;
+      a.mn[c] = dkey(cvt_from(mn[c], S));
+      a.mx[c] = dkey(cvt_from(mx[c], S));
+    }
+    a.mn[2] = zn;
+    a.mx[2] = zx;
+  }
+};
+
+// Copies the potential and line density the kick reads into the block's
+// shared memory (threads t0.. of the block): KF 1 as fixed-point pairs made
+// from the FP64 values at the scales the kick constants use.
+template <int KF>
+__device__ __forceinline__ void fill_kick_grids(const KickArgs& kick, unsigned char* s_raw, int t0) {
+  const int ng = kick.nx * kick.ny;
+  if (KF == 1) {
+    const int sphi = scale_bits(kick.st->phi_absmax), slam = scale_bits(kick.st->lam_absmax);
+    double* sd = reinterpret_cast<double*>(s_raw);  // the FP64 values land in place and become integers there
+    copy_smem_async(sd, kick.phi, ng,
+                    [sphi](double v) { return __longlong_as_double(fx_pair(phi_fixed(v, sphi))); }, t0);
+    copy_smem_async(sd + ng, kick.lam, kick.nz,
+                    [slam](double v) { return __longlong_as_double(fx_pair(phi_fixed(v, slam))); }, t0);
+  } else {
+    float* s = reinterpret_cast<float*>(s_raw);
+    copy_smem_async(s, kick.phi_f, ng, [](float v) { return v; }, t0);
+    copy_smem_async(s + ng, kick.lam_f, kick.nz, [](float v) { return v; }, t0);
+  }
+}
+
 // KF: 0 no kick, 1 plain kick, 2 fp32 kick.  EXT: accumulate extrema.
-// Blocks blk = 0..nblk-1 share the bunch's particles.
+// Blocks blk = 0..nblk-1 share the bunch's particles.  The FP64 pass: the
+// first of a run, and those whose maps or kick (2.5Drb) have no fixed-point
+// form.
 template <int KF, bool EXT, bool KSMEM>
 __device__ __forceinline__ void pass_body(double* __restrict__ cx, double* __restrict__ cxp,
                                           double* __restrict__ cy, double* __restrict__ cyp,
@@ -90,34 +255,22 @@ __device__ __forceinline__ void pass_body(double* __restrict__ cx, double* __res
     __shared__ KickFix s_kf;
     if (threadIdx.x == 0) kick_consts_into(&s_k, KF == 1 ? &s_kf : nullptr, kick);
     if (KSMEM) {
-      const int ng = kick.nx * kick.ny, t0 = blockDim.x > 64 ? 32 : 0;
-      if (KF == 1) {
-        // fixed-point copy converted here from the FP64 potential, at the
-        // scales the kick constants use
-        const int sphi = scale_bits(kick.st->phi_absmax), slam = scale_bits(kick.st->lam_absmax);
-        long long* s = reinterpret_cast<long long*>(s_raw);
-        // the FP64 values land in place and become 64-bit integers there
-        double* sd = reinterpret_cast<double*>(s_raw);
-        copy_smem_async(sd, kick.phi, ng,
-                        [sphi](double v) { return __longlong_as_double(phi_fixed(v, sphi)); }, t0);
-        copy_smem_async(sd + ng, kick.lam, kick.nz,
-                        [slam](double v) { return __longlong_as_double(phi_fixed(v, slam)); }, t0);
-        P = s;
-        Lm = s + ng;
-      } else {
-        float* s = reinterpret_cast<float*>(s_raw);
-        copy_smem_async(s, kick.phi_f, ng, [](float v) { return v; }, t0);
-        copy_smem_async(s + ng, kick.lam_f, kick.nz, [](float v) { return v; }, t0);
-        Pf = s;
-        Lf = s + ng;
-      }
+      fill_kick_grids<KF>(kick, s_raw, blockDim.x > 64 ? 32 : 0);
+      P = reinterpret_cast<const long long*>(s_raw);
+      Lm = P + kick.nx * kick.ny;
+      Pf = reinterpret_cast<const float*>(s_raw);
+      Lf = Pf + kick.nx * kick.ny;
     }
     __syncthreads();
     k = s_k;
     if (KF == 1) kf = s_kf;
   }
   ExtAcc acc;
-  if (EXT) acc.init();
+  MagAcc mag;
+  if (EXT) {
+    acc.init();
+    mag.init();
+  }
   for (int i = blk * blockDim.x + threadIdx.x; i < n; i += nblk * blockDim.x) {
     Part p;
     p.x = cx[i]; p.xp = cxp[i]; p.y = cy[i]; p.yp = cyp[i]; p.z = cz[i]; p.dE = cdE[i];
@@ -139,7 +292,14 @@ __device__ __forceinline__ void pass_body(double* __restrict__ cx, double* __res
     }
     if (KF == 2 && !k.skip && bnd_inside(kick.bnd, p.x, p.y)) kick_fp32(k, Pf, Lf, p.x, p.y, p.z, p.xp, p.yp);
     apply_ops<ORBIT_SOFT_MUL>(p, ops, a, b, m);
-    if (EXT) acc.add(p.x, p.y, p.z);
+    if (EXT) {
+      acc.add(p.x, p.y, p.z);
+      if (sa.mag) {
+        mag.bound(p.xp, p.yp);
+        mag.em = max(mag.em, MagAcc::hi(p.dE));
+        if (i < nblk * (int)blockDim.x) mag.sample(p.x, p.xp, p.y, p.yp);
+      }
+    }
     if (km & KNL_STORE) {
       ensure_knl<ORBIT_SOFT_MUL & 1>(p, m);
       knl_buf[i] = p.knl;
@@ -147,7 +307,126 @@ __device__ __forceinline__ void pass_body(double* __restrict__ cx, double* __res
     cx[i] = p.x; cxp[i] = p.xp; cy[i] = p.y; cyp[i] = p.yp; cz[i] = p.z; cdE[i] = p.dE;
   }
   // the last block sets up the grids of the next kick
-  if (EXT) ext_commit_and_setup(acc, ext_st, status, sa, nblk);
+  if (EXT) {
+    if (sa.mag) mag_block_commit(mag, ext_st);
+    ext_commit_and_setup(acc, ext_st, status, sa, nblk);
+  }
+}
+
+// The pass in fixed point: maps that all have a fixed-point form, dE and
+// 1/(1+dp_p) unchanged, the plain form's kick.  A pass whose magnitudes or
+// constants do not fit (FxPass::ok, the same in every block) goes particle by
+// particle through the FP64 routines.
+//
+// Bound by the issue of integer instructions: 777 a particle for a kick and a
+// drift, about 1300 with two half quadrupoles and their fringes, at half an
+// instruction a clock per sub-partition with 5 warps there (512, 640 and 768
+// threads are within 3% of one another).  At 1e6 particles, 128 x 128 x 64, a
+// FODO segment: 53 us against 140 us of the FP64 pass; at 16e6 particles,
+// 256 x 256 x 64, ring segments: 2.0 ms against 4.3 ms.
+//
+// The FP32 form keeps the FP64 pass: a rounding of its fields that flips
+// moves the whole potential by 5e-8, so coordinates that differ in the last
+// bit give beams that differ at the form's own error, 2e-5 after 16 kicks.
+template <bool EXT, bool KSMEM>
+__device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __restrict__ cxp,
+                                             double* __restrict__ cy, double* __restrict__ cyp,
+                                             double* __restrict__ cz, const double* __restrict__ cdE, int n,
+                                             const DevOp* __restrict__ ops, int a, int b, const MapCtx& m,
+                                             const KickArgs& kick, ScState* ext_st, unsigned* status,
+                                             const SetupArgs& sa, const double* __restrict__ knl_buf,
+                                             const PassPrep* __restrict__ prep, int blk, int nblk) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  __shared__ FxFallback s_f;
+  __shared__ PassPrep s_prep;
+  FxPass& s_fx = s_prep.fx;
+  // warp 0 takes the constants made beside the solve and adds what hangs on
+  // the potential's maximum while warps 1.. fill the block's copy of the
+  // potential and the line density; one barrier completes both
+  if (threadIdx.x < 32) {
+    load_prep(prep, kick.st, b - a, &s_prep);
+    if (threadIdx.x == 0) {
+      const size_t ng = (size_t)kick.nx * kick.ny;
+      s_f.P = KSMEM ? reinterpret_cast<const long long*>(s_raw) : kick.phi_fix;
+      s_f.Lm = KSMEM ? s_f.P + ng : kick.lam_fix;
+      s_f.c[0] = cx; s_f.c[1] = cxp; s_f.c[2] = cy; s_f.c[3] = cyp; s_f.c[4] = cz;
+      s_f.k = &s_prep.k; s_f.kf = &s_prep.kf;
+      s_f.dE = cdE; s_f.knl = knl_buf; s_f.kick = &kick; s_f.m = &m; s_f.ops = ops; s_f.a = a; s_f.b = b;
+      for (int c = 0; c < 3; ++c) { s_f.mn[c] = ~0ull; s_f.mx[c] = 0ull; }
+      s_f.pm = s_f.sx = s_f.sp = s_f.n = 0u;
+      s_f.bad = 0;
+    }
+  }
+  if (KSMEM) fill_kick_grids<1>(kick, s_raw, blockDim.x > 64 ? 32 : 0);
+  __syncthreads();
+  const long long* P = KSMEM ? reinterpret_cast<const long long*>(s_raw) : kick.phi_fix;
+  const long long* Lm = KSMEM ? P + (size_t)kick.nx * kick.ny : kick.lam_fix;
+  const bool fixed = s_fx.ok != 0, bound = kick.bnd.type >= 0;
+  const fx::Scales s = s_fx.s;
+  ExtFx ext;
+  MagAcc mag;
+  if (EXT) {
+    ext.init();
+    mag.init();
+  }
+  for (int i = blk * blockDim.x + threadIdx.x; i < n; i += nblk * blockDim.x) {
+    bool ok = fixed;
+    fx::Part t;
+    if (ok) {
+      const double x = cx[i], xp = cxp[i], y = cy[i], yp = cyp[i], dE = cdE[i];
+      const double knl = knl_buf[i];  // as an earlier pass of this run computed it from the same dE
+      const double dp = __dmul_rn(dE, m.dp_p_coeff);
+      t.z = cz[i];
+      t.x = cvt_to(x, s.x);
+      t.p = cvt_to(xp, s.p);
+      t.y = cvt_to(y, s.x);
+      t.r = cvt_to(yp, s.p);
+      if (s_fx.check) {
+        auto inside = [](double v, int lim) { return (__double2hiint(v) & 0x7fffffff) <= lim; };
+        ok = inside(x, s_fx.limx) & inside(y, s_fx.limx) & inside(xp, s_fx.limp) & inside(yp, s_fx.limp) &
+             inside(dp, s_fx.limd);
+      }
+      if (ok && (!bound || bnd_inside(kick.bnd, x, y))) {
+        ok = kick_fx(s_fx, kick.nx, P, Lm, t);
+      }
+      fx::part_init(t, fx::kappa_of(knl), cvt_to(dp, s.k), s.k);
+    }
+    if (!ok) {
+      pass_particle<EXT>(&s_f, i, i < nblk * (int)blockDim.x);
+      continue;
+    }
+    fx::apply(t, s_fx.op, s_fx.n, s);
+    const double x = cvt_from(t.x, s.x), xp = cvt_from(t.p, s.p), y = cvt_from(t.y, s.x), yp = cvt_from(t.r, s.p);
+    const double z = t.z + cvt_from(t.d, s.d);
+    if (EXT) {
+      ext.add(t.x, t.y, z);
+      mag.bound(xp, yp);
+      if (i < nblk * (int)blockDim.x) mag.sample(x, xp, y, yp);  // the thread's first particle
+    }
+    cx[i] = x; cxp[i] = xp; cy[i] = y; cyp[i] = yp; cz[i] = z;
+  }
+  // the last block sets up the grids of the next kick
+  if (EXT) {
+    __syncthreads();  // the fallback's shared extrema
+    ExtAcc acc;
+    acc.init();
+    ext.join(acc, s.x);
+    if (threadIdx.x == 0) {
+      for (int c = 0; c < 3; ++c) {
+        acc.mn[c] = min(acc.mn[c], s_f.mn[c]);
+        acc.mx[c] = max(acc.mx[c], s_f.mx[c]);
+      }
+      acc.bad = s_f.bad != 0;
+      mag.pm = max(mag.pm, s_f.pm);
+      // dE is unchanged; without magnitudes before, none are claimed
+      mag.em = kick.st->mag.pmax ? kick.st->mag.emax : 0x7fefffffu;
+      mag.sx += s_f.sx;
+      mag.sp += s_f.sp;
+      mag.n += s_f.n;
+    }
+    if (sa.mag) mag_block_commit(mag, ext_st);
+    ext_commit_and_setup(acc, ext_st, status, sa, nblk);
+  }
 }
 
 template <int KF, bool EXT, bool KSMEM>
@@ -155,13 +434,28 @@ __global__ void __launch_bounds__(ORBIT_PASS_THREADS) k_pass(double* __restrict_
                                               double* __restrict__ cy, double* __restrict__ cyp,
                                               double* __restrict__ cz, double* __restrict__ cdE, int n,
                                               const DevOp* __restrict__ ops, int a, int b, MapCtx m,
-                                              KickArgs kick, ScState* ext_st, unsigned* status, SetupArgs sa,
+                                              KickArgs kick, ScState* ext_st, unsigned* status,
+                                              const __grid_constant__ SetupArgs sa,
                                               double* __restrict__ knl_buf, int km) {
   pass_body<KF, EXT, KSMEM>(cx, cxp, cy, cyp, cz, cdE, n, ops, a, b, m, kick, ext_st, status, sa, knl_buf, km,
                             blockIdx.x, gridDim.x);
 }
 
-// The same pass for the members of a batch class; each block finds its
+template <bool EXT, bool KSMEM>
+__global__ void __launch_bounds__(ORBIT_FX_THREADS) k_pass_fx(double* __restrict__ cx, double* __restrict__ cxp,
+                                              double* __restrict__ cy, double* __restrict__ cyp,
+                                              double* __restrict__ cz, const double* __restrict__ cdE, int n,
+                                              const DevOp* __restrict__ ops, int a, int b,
+                                              const __grid_constant__ MapCtx m,
+                                              const __grid_constant__ KickArgs kick, ScState* ext_st,
+                                              unsigned* status, const __grid_constant__ SetupArgs sa,
+                                              const double* __restrict__ knl_buf,
+                                              const PassPrep* __restrict__ prep) {
+  pass_fx_body<EXT, KSMEM>(cx, cxp, cy, cyp, cz, cdE, n, ops, a, b, m, kick, ext_st, status, sa, knl_buf,
+                               prep, blockIdx.x, gridDim.x);
+}
+
+// The same passes for the members of a batch class; each block finds its
 // member in the block table.
 template <int KF, bool EXT, bool KSMEM>
 __global__ void __launch_bounds__(ORBIT_PASS_THREADS) kb_pass(const PassJob* __restrict__ jobs,
@@ -174,6 +468,17 @@ __global__ void __launch_bounds__(ORBIT_PASS_THREADS) kb_pass(const PassJob* __r
                             J.status, J.sa, J.knl, km, blockIdx.x - mb.x, mb.y);
 }
 
+template <bool EXT, bool KSMEM>
+__global__ void __launch_bounds__(ORBIT_FX_THREADS) kb_pass_fx(const PassJob* __restrict__ jobs,
+                                               const unsigned short* __restrict__ blk_job,
+                                               const int2* __restrict__ mblk, int a, int b) {
+  const int j = blk_job[blockIdx.x];
+  const PassJob& J = jobs[j];
+  const int2 mb = mblk[j];
+  pass_fx_body<EXT, KSMEM>(J.c[0], J.c[1], J.c[2], J.c[3], J.c[4], J.c[5], J.n, J.ops, a, b, J.m, J.ka, J.ext,
+                              J.status, J.sa, J.knl, J.prep, blockIdx.x - mb.x, mb.y);
+}
+
 // Shared-memory limits are raised once, outside any stream capture.
 static int init_pass_attrs() {
   static bool done = false;
@@ -184,6 +489,10 @@ static int init_pass_attrs() {
   ORBIT_CUDA(cudaFuncSetAttribute(k_pass<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));
   ORBIT_CUDA(cudaFuncSetAttribute(kb_pass<1, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));
   ORBIT_CUDA(cudaFuncSetAttribute(kb_pass<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));
+  ORBIT_CUDA(cudaFuncSetAttribute(k_pass_fx<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));
+  ORBIT_CUDA(cudaFuncSetAttribute(k_pass_fx<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));
+  ORBIT_CUDA(cudaFuncSetAttribute(kb_pass_fx<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));
+  ORBIT_CUDA(cudaFuncSetAttribute(kb_pass_fx<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem));
   done = true;
   return ORBIT_OK;
 }
@@ -191,8 +500,8 @@ static int init_pass_attrs() {
 template <int KF, bool EXT, bool KSMEM>
 static int launch_pass(orbit_bunch_t* bu, cudaStream_t s, size_t smem, const DevOp* ops, int a, int b,
                        const MapCtx& m, const KickArgs& ka, ScState* ext, const SetupArgs& sa, double* knl_buf,
-                       int km) {
-  int threads = ORBIT_PASS_THREADS;
+                       int km, bool fixed, const PassPrep* prep) {
+  int threads = fixed ? ORBIT_FX_THREADS : ORBIT_PASS_THREADS;
   int bps = KSMEM ? (int)(kPassSmem / (smem > 0 ? smem : 1)) : 4;
   if (bps < 1) bps = 1;
   if (bps > 4) bps = 4;
@@ -200,6 +509,16 @@ static int launch_pass(orbit_bunch_t* bu, cudaStream_t s, size_t smem, const Dev
   int need = (bu->n + threads - 1) / threads;
   if (need < blocks) blocks = need < 1 ? 1 : need;
   ORBIT_PB(KF == 0 ? "pass_maps" : "pass_kick_maps", s);
+  if constexpr (KF == 1) {
+    if (fixed) {
+      k_pass_fx<EXT, KSMEM><<<blocks, threads, KSMEM ? smem : 0, s>>>(
+          bu->coord(0), bu->coord(1), bu->coord(2), bu->coord(3), bu->coord(4), bu->coord(5), bu->n, ops, a, b, m,
+          ka, ext, bu->d_status, sa, knl_buf, prep);
+      ORBIT_PE(s);
+      ORBIT_LAUNCH_CHECK("k_pass_fx");
+      return ORBIT_OK;
+    }
+  }
   k_pass<KF, EXT, KSMEM><<<blocks, threads, KSMEM ? smem : 0, s>>>(
       bu->coord(0), bu->coord(1), bu->coord(2), bu->coord(3), bu->coord(4), bu->coord(5), bu->n, ops, a, b, m, ka,
       ext, bu->d_status, sa, knl_buf, km);
@@ -211,7 +530,7 @@ static int launch_pass(orbit_bunch_t* bu, cudaStream_t s, size_t smem, const Dev
 size_t batch_pass_smem_limit() { return kPassSmem; }
 
 int batch_enqueue_pass(const PassJob* jobs, const BlockMap& bm, int threads, int kf, bool ext, bool ksmem,
-                       size_t smem, int a, int b, int km, cudaStream_t s, const char* tag) {
+                       size_t smem, int a, int b, int km, bool fixed, cudaStream_t s, const char* tag) {
   int arc = init_pass_attrs();
   if (arc) return arc;
   const int nb = bm.nblk;
@@ -219,6 +538,15 @@ int batch_enqueue_pass(const PassJob* jobs, const BlockMap& bm, int threads, int
   if (kf == 0) {
     if (ext) kb_pass<0, true, false><<<nb, threads, 0, s>>>(jobs, bm.blk_job, bm.mblk, a, b, km);
     else kb_pass<0, false, false><<<nb, threads, 0, s>>>(jobs, bm.blk_job, bm.mblk, a, b, km);
+  } else if (fixed) {
+    const int t = ORBIT_FX_THREADS;
+    if (ksmem) {
+      if (ext) kb_pass_fx<true, true><<<nb, t, smem, s>>>(jobs, bm.blk_job, bm.mblk, a, b);
+      else kb_pass_fx<false, true><<<nb, t, smem, s>>>(jobs, bm.blk_job, bm.mblk, a, b);
+    } else {
+      if (ext) kb_pass_fx<true, false><<<nb, t, 0, s>>>(jobs, bm.blk_job, bm.mblk, a, b);
+      else kb_pass_fx<false, false><<<nb, t, 0, s>>>(jobs, bm.blk_job, bm.mblk, a, b);
+    }
   } else if (ksmem) {
     if (ext) kb_pass<1, true, true><<<nb, threads, smem, s>>>(jobs, bm.blk_job, bm.mblk, a, b, km);
     else kb_pass<1, false, true><<<nb, threads, smem, s>>>(jobs, bm.blk_job, bm.mblk, a, b, km);
@@ -284,6 +612,8 @@ static int enqueue_pass(orbit_bunch_t* bu, cudaStream_t s, const DevOp* ops, Seg
     ksm = kc->smem_kick && smem <= (size_t)kPassSmem;  // else the kick reads phi_fix, converted by the solve
   }
   if (!kc && !ec && seg.a == seg.b) return ORBIT_OK;  // nothing to do
+  const bool fixed = fixed_pass(seg, kc && kc->form == ORBIT_FORM_PLAIN && !kc->rb, km);
+  const PassPrep* prep = kc ? kc->d_prep : nullptr;
   ScState* ext = ec ? ec->d_st : nullptr;
   bool e = ext != nullptr;
   SetupArgs sa;
@@ -293,18 +623,18 @@ static int enqueue_pass(orbit_bunch_t* bu, cudaStream_t s, const DevOp* ops, Seg
     if (ec_here) sa.cond = sc_green_cond(ec, s, true);
   }
   int rc;
-  if (kf == 0) rc = e ? launch_pass<0, true, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km)
-                      : launch_pass<0, false, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km);
+  if (kf == 0) rc = e ? launch_pass<0, true, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep)
+                      : launch_pass<0, false, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep);
   else if (kf == 1) {
-    if (ksm) rc = e ? launch_pass<1, true, true>(bu, s, smem, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km)
-                    : launch_pass<1, false, true>(bu, s, smem, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km);
-    else rc = e ? launch_pass<1, true, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km)
-                : launch_pass<1, false, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km);
+    if (ksm) rc = e ? launch_pass<1, true, true>(bu, s, smem, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep)
+                    : launch_pass<1, false, true>(bu, s, smem, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep);
+    else rc = e ? launch_pass<1, true, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep)
+                : launch_pass<1, false, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep);
   } else {
-    if (ksm) rc = e ? launch_pass<2, true, true>(bu, s, smem, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km)
-                    : launch_pass<2, false, true>(bu, s, smem, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km);
-    else rc = e ? launch_pass<2, true, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km)
-                : launch_pass<2, false, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km);
+    if (ksm) rc = e ? launch_pass<2, true, true>(bu, s, smem, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep)
+                    : launch_pass<2, false, true>(bu, s, smem, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep);
+    else rc = e ? launch_pass<2, true, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep)
+                : launch_pass<2, false, false>(bu, s, 0, ops, seg.a, seg.b, m, ka, ext, sa, knl_buf, km, fixed, prep);
   }
   if (rc == ORBIT_OK) ++*nl;
   return rc;
@@ -335,17 +665,21 @@ int compile(orbit_program_t* p, orbit_bunch_t* bu, Plan& plan) {
   auto lengthwise = [](int code) {
     return code == ORBIT_OP_DRIFT ? 1 : (code == ORBIT_OP_QUAD2 || code == ORBIT_OP_BEND2) ? 2 : 0;
   };
-  auto emit = [&](int a, int b) -> Seg {
+  auto emit = [&](int a, int b, bool start) -> Seg {
     Seg s;
+    if (start) dev.push_back(DevOp{});  // the segment's start entry (fx::compile_segment)
     s.a = (int)dev.size();
     s.dE = false;
     for (int k = a; k < b; ++k) {
       DevOp d;
       double adv = 0.0;
-      if (!compile_op(p->ops[k], bu->sync, d, &adv)) return Seg{-1, -1, false};
+      if (!compile_op(p->ops[k], bu->sync, d, &adv)) return Seg{-1, -1, false, false};
       p->time_adv[k] = adv;
       if (d.code == ORBIT_OP_WEDGEROT || (d.code == ORBIT_OP_KICK && d.c[2] != 0.)) s.dE = true;
       if (d.code == 0) continue;
+      if (bu->sync.charge == 0. &&
+          (d.code == ORBIT_OP_MULTP || d.code == ORBIT_OP_MPFRIN || d.code == ORBIT_OP_MPFROUT))
+        continue;  // no effect on a neutral bunch (teapotbase.cc:340, 397, 510)
       if (lengthwise(d.code) && (int)dev.size() > s.a && lengthwise(dev.back().code) == lengthwise(d.code)) {
         dev.back().c[0] += d.c[0];
         continue;
@@ -356,20 +690,33 @@ int compile(orbit_program_t* p, orbit_bunch_t* bu, Plan& plan) {
     return s;
   };
   for (auto& so : seg_ops) {
-    Seg s = emit(so.first, so.second);
+    Seg s = emit(so.first, so.second, true);
     if (s.a < 0) return set_error(ORBIT_ERR_ARG, "orbit_program: bad op parameters");
     plan.segs.push_back(s);
   }
   Seg w;
-  w.a = (int)dev.size();
   {
-    Seg s1 = emit(seg_ops.back().first, seg_ops.back().second);
-    Seg s2 = emit(seg_ops.front().first, seg_ops.front().second);
+    Seg s1 = emit(seg_ops.back().first, seg_ops.back().second, true);
+    w.a = s1.a;
+    Seg s2 = emit(seg_ops.front().first, seg_ops.front().second, false);
     if (s1.a < 0 || s2.a < 0) return set_error(ORBIT_ERR_ARG, "orbit_program: bad op parameters");
   }
   w.b = (int)dev.size();
   w.dE = plan.segs.back().dE || plan.segs.front().dE;
   plan.wrap = w;
+  const double g2 = make_ctx(bu->sync).gamma2i;
+  auto mark = [&](Seg& sg) {
+    fx::compile_segment(&dev[sg.a - 1], sg.b - sg.a, g2);
+    bool moves = false;
+    sg.fx = sg.b - sg.a < fx::kMaxOps;
+    for (int k = sg.a; k < sg.b; ++k) {
+      sg.fx = sg.fx && fx::supported(dev[k]);
+      moves = moves || fx::moves_x(dev[k]);
+    }
+    sg.fx = sg.fx && moves;  // x and y are rewritten: thin kicks alone leave them as they are
+  };
+  for (Seg& sg : plan.segs) mark(sg);
+  mark(plan.wrap);
   if (p->knl_n < (size_t)bu->n) {
     if (p->d_knl) { cudaFree(p->d_knl); p->d_knl = nullptr; }
     p->knl_n = 0;
@@ -430,19 +777,25 @@ static int enqueue_turn(orbit_program_t* p, orbit_bunch_t* bu, cudaStream_t s, c
     if (rc) return rc;
   }
   for (int i = 0; i < nsc; ++i) {
-    rc = sc_enqueue_kick(calc_of(i), bu, len_of(i), s, false, false, nl, pipe_of(i), bnd_of(i));
-    if (rc) return rc;
-    bool last = (i == nsc - 1);
-    if (!last) {
-      rc = enqueue_pass(bu, s, ops, plan.segs[i + 1], m, calc_of(i), len_of(i), bnd_of(i), calc_of(i + 1),
-                        bnd_of(i + 1), true, knl, km_of(plan.segs[i + 1], true, calc_of(i)), nl);
-    } else if (wrap) {
-      rc = enqueue_pass(bu, s, ops, plan.wrap, m, calc_of(i), len_of(i), bnd_of(i), calc_of(0), bnd_of(0), false,
-                        knl, km_of(plan.wrap, true, calc_of(i)), nl);
-    } else {
-      rc = enqueue_pass(bu, s, ops, plan.segs[nsc], m, calc_of(i), len_of(i), bnd_of(i), nullptr, nullptr, false,
-                        knl, km_of(plan.segs[nsc], true, calc_of(i)), nl);
+    const bool last = (i == nsc - 1);
+    const Seg& sg = !last ? plan.segs[i + 1] : (wrap ? plan.wrap : plan.segs[nsc]);
+    orbit_sc2p5d_t* kc = calc_of(i);
+    const int km = km_of(sg, true, kc);
+    PrepJob job;
+    std::memset(&job, 0, sizeof(job));
+    if (fixed_pass(sg, kc->form == ORBIT_FORM_PLAIN && !kc->rb, km)) {
+      job.ops = ops; job.a = sg.a; job.b = sg.b;
+      job.dp_p_coeff = m.dp_p_coeff;
+      job.host_factor = sc_host_factor(bu->sync, len_of(i));
+      job.out = kc->d_prep;
     }
+    rc = sc_enqueue_kick(kc, bu, len_of(i), s, false, false, nl, pipe_of(i), bnd_of(i), &job);
+    if (rc) return rc;
+    // the last pass of a turn that another one follows also applies M_0 and
+    // scans for the next turn's first kick
+    orbit_sc2p5d_t* ec = !last ? calc_of(i + 1) : (wrap ? calc_of(0) : nullptr);
+    rc = enqueue_pass(bu, s, ops, sg, m, kc, len_of(i), bnd_of(i), ec, !last ? bnd_of(i + 1) : bnd_of(0), !last, knl,
+                      km, nl);
     if (rc) return rc;
   }
   return ORBIT_OK;

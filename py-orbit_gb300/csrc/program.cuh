@@ -39,6 +39,7 @@ namespace orbit {
 struct Seg {
   int a, b;
   bool dE;  // an op of the segment changes dE (kick with dE, wedgerotate)
+  bool fx = false;  // every map has a fixed-point form (fixmap.cuh)
 };
 
 struct Plan {
@@ -51,6 +52,11 @@ struct Plan {
 // (it changes only with dE): km & KNL_STORE writes it at the end of the
 // pass, km & KNL_LOAD reads it instead of dividing.
 enum { KNL_LOAD = 1, KNL_STORE = 2 };
+
+// A pass that runs in fixed point (where the bunch's magnitudes then allow):
+// it starts with a transverse kick, its maps all have a fixed-point form and
+// it neither computes nor changes 1/(1+dp_p).
+inline bool fixed_pass(const Seg& sg, bool kick, int km) { return kick && sg.fx && km == KNL_LOAD; }
 
 // Builds the device op array of the program for the bunch's reference
 // particle: all non-SC ops of the turn in order, then the wrap segment.

@@ -10,6 +10,7 @@
 #include "fft.cuh"
 #include "sc2p5d.cuh"
 #include "sc_device.cuh"
+#include "passprep.cuh"
 #include "batch.cuh"
 
 namespace orbit {
@@ -49,7 +50,8 @@ double sc_rb_long_factor(const orbit_sync_t& s, double length) {
 // Extrema scan; the last block sets up the grids for the kick.  The
 // accumulation grids start at zero: the kernels that read them clear them.
 __global__ void k_extrema(const double* __restrict__ x, const double* __restrict__ y,
-                          const double* __restrict__ z, int n, ScState* st, unsigned* status, SetupArgs sa) {
+                          const double* __restrict__ z, int n, ScState* st, unsigned* status,
+                          const __grid_constant__ SetupArgs sa) {
   ExtAcc a;
   a.init();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a.add(x[i], y[i], z[i]);
@@ -101,6 +103,7 @@ __device__ __noinline__ void finalize_block(ScState* st, G* zacc, int nz, double
     if (reset_dirty) st->green_dirty = 0;
     st->n_kicks += 1;
   }
+  if (threadIdx.x == blockDim.x - 1) st->scale = log(st->scale_arg);  // PoissonSolverFFT2D.cc:213
   __shared__ double s_part[32];
   double iq = st->inv_qscale;
   double acc = 0.0;
@@ -191,12 +194,17 @@ __device__ __forceinline__ void rows_fwd_body(ScState* st, void* src, double* rh
                                               int nrows, int ncols, int H, int gate, void* zacc, int nz,
                                               double* lam, float* lam_f, int blk, int nblk,
                                               typename CT<T>::t* sa = nullptr,
-                                              const typename CT<T>::t* stw_in = nullptr, bool reset_dirty = true) {
+                                              const typename CT<T>::t* stw_in = nullptr, bool reset_dirty = true,
+                                              const PrepJob* prep = nullptr) {
   typedef typename CT<T>::t C;
   if (SRC == 0 && gate && !st->green_dirty) return;
   if (st->skip) return;
   if (SRC == 1 && blk == nblk - 1) {
     finalize_block(st, (unsigned long long*)zacc, nz, lam, lam_f, reset_dirty);
+    if (prep && prep->out) {
+      __syncthreads();
+      if (threadIdx.x < 32) prep_pass(*prep, st, nrows, ncols, nz, nullptr, 0, 0, nullptr);
+    }
     return;
   }
   extern __shared__ unsigned char smem_raw[];
@@ -281,9 +289,10 @@ __device__ __forceinline__ void rows_fwd_body(ScState* st, void* src, double* rh
 template <typename T, int SRC>
 __global__ void k_rows_fwd(ScState* st, void* src, double* rho_out, typename CT<T>::t* hat,
                            const typename CT<T>::t* __restrict__ tw, FftPlan pl, int nrows, int ncols, int H,
-                           int gate, void* zacc, int nz, double* lam, float* lam_f) {
+                           int gate, void* zacc, int nz, double* lam, float* lam_f,
+                           const __grid_constant__ PrepJob prep) {
   rows_fwd_body<T, SRC>(st, src, rho_out, hat, tw, pl, nrows, ncols, H, gate, zacc, nz, lam, lam_f, blockIdx.x,
-                        gridDim.x);
+                        gridDim.x, nullptr, nullptr, true, &prep);
 }
 
 // Column transforms along x (length N = nx2), one column k per block.
@@ -332,7 +341,7 @@ __device__ __forceinline__ void cols_body(ScState* st, typename CT<T>::t* hat, t
     if (k == 0 && threadIdx.x == 0) st->n_green += 1;
     return;
   }
-  double s = st->scale;
+  const double s = CG ? __ldcg(&st->scale) : st->scale;
   for (int r = threadIdx.x; r < N; r += blockDim.x) {
     C g = ldx<CG>(green + (size_t)k * N + r);
     T gr;
@@ -459,6 +468,7 @@ struct ConvArgs {
   double denom;             // 1 / (nx2 ny2)
   long long wait_polls;     // barrier wait limit
   int withhold;             // test hook: this block skips the first barrier (-1: none)
+  PrepJob prep;             // the pass that follows
 };
 
 // Grid-wide barrier on a counter zeroed by the kick's set-up: every block
@@ -471,21 +481,7 @@ __device__ __forceinline__ bool conv_barrier(unsigned* cnt, unsigned nblk, long 
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(cnt, 1u);
-    int ok = 1;
-    long long i = 0;
-    for (;;) {
-      unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
-      if (v >= nblk) break;
-      if (++i > polls) {
-        ok = 0;
-        break;
-      }
-      __nanosleep(32);
-    }
-    if (!ok) atomicOr(status, (unsigned)ST_SYNC);
-    __threadfence();
-    s_ok = ok;
+    s_ok = counter_wait(cnt, nblk, polls, status);
   }
   __syncthreads();
   return s_ok != 0;
@@ -496,7 +492,7 @@ __device__ __forceinline__ bool conv_barrier(unsigned* cnt, unsigned nblk, long 
 // square power-of-two doubled grid nx2 = ny2 = 2^LOGN, transforms
 // specialised at compile time (block_fft_fixed); 0: any supported size.
 template <typename T, int LOGN>
-__global__ void k_conv_fused(ConvArgs A) {
+__global__ void k_conv_fused(const __grid_constant__ ConvArgs A) {
   typedef typename CT<T>::t C;
   constexpr int SRC = 1;  // both forms deposit in fixed point
   extern __shared__ unsigned char smem_raw[];
@@ -513,9 +509,22 @@ __global__ void k_conv_fused(ConvArgs A) {
   C* hat = (C*)A.hat;
   C* green = (C*)A.green;
   C* gscr = (C*)A.gscr;
+  // an extra block makes the constants of the pass that follows; it has
+  // nothing the others wait for and arrives at both barriers at once
+  const int nw = gridDim.x - (A.prep.out ? 1 : 0);
+  if ((int)blockIdx.x == nw) {
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0) {
+        atomicAdd(&st->conv_bar[0], 1u);
+        atomicAdd(&st->conv_bar[1], 1u);
+      }
+      prep_pass(A.prep, st, A.nx, A.ny, A.nz, &st->conv_bar[0], gridDim.x, A.wait_polls, A.status);
+    }
+    return;
+  }
   // phase 1: deposit rows (+ the finalization item), Green rows
   const int nrp = (A.nx + 1) / 2, ngp = dirty ? (A.nx + 2) / 2 : 0;
-  for (int it = blockIdx.x; it < nrp + 1 + ngp; it += gridDim.x) {
+  for (int it = blockIdx.x; it < nrp + 1 + ngp; it += nw) {
     if (it <= nrp)
       rows_fwd_body<T, SRC, LOGN>(st, A.src, A.rho, hat, nullptr, A.ply, A.nx, A.ny, A.H, 1, A.zacc, A.nz, A.lam,
                                   A.lam_f, it, nrp + 1, a, sty, false);
@@ -529,7 +538,7 @@ __global__ void k_conv_fused(ConvArgs A) {
   if (blockIdx.x == 0 && threadIdx.x == 0 && dirty) st->green_dirty = 0;
   // phase 2: per column, the Green column (when rebuilt), then the deposit's
   // forward transform, the multiply and the backward transform
-  for (int k = blockIdx.x; k < A.H; k += gridDim.x) {
+  for (int k = blockIdx.x; k < A.H; k += nw) {
     if (dirty) {
       cols_body<T, 0, true, LOGN>(st, gscr, green, nullptr, A.plx, A.nx2, A.H, A.ny2, 0, k, a, stx);
       __syncthreads();
@@ -539,7 +548,7 @@ __global__ void k_conv_fused(ConvArgs A) {
   }
   if (!conv_barrier(&st->conv_bar[1], gridDim.x, A.wait_polls, A.status)) return;
   // phase 3: backward rows onto phi
-  for (int it = blockIdx.x; it < nrp; it += gridDim.x) {
+  for (int it = blockIdx.x; it < nrp; it += nw) {
     rows_inv_body<T, true, LOGN>(st, hat, nullptr, A.ply, A.nx, A.ny, A.H, A.denom, A.phi, A.phi_f, it, a, sty);
     __syncthreads();
   }
@@ -554,8 +563,8 @@ __device__ __forceinline__ void phi_fix_body(const ScState* st, const double* __
   if (st->skip) return;
   int sphi = scale_bits(st->phi_absmax), slam = scale_bits(st->lam_absmax);
   int i = blk * blockDim.x + threadIdx.x;
-  if (i < ng) phi_fix[i] = phi_fixed(phi[i], sphi);
-  if (i < nz) lam_fix[i] = phi_fixed(lam[i], slam);
+  if (i < ng) phi_fix[i] = fx_pair(phi_fixed(phi[i], sphi));
+  if (i < nz) lam_fix[i] = fx_pair(phi_fixed(lam[i], slam));
 }
 
 __global__ void k_phi_fix(const ScState* st, const double* __restrict__ phi, const double* __restrict__ lam,
@@ -811,8 +820,8 @@ __global__ void k_kick_plain(const double* __restrict__ x, double* __restrict__ 
   const long long* Lm = lam_fix;
   if (SMEM) {
     // the shared copy is converted here; phi_fix, lam_fix are not read
-    for (int i = threadIdx.x; i < nx * ny; i += blockDim.x) s_phix[i] = phi_fixed(phi[i], kf.sphi);
-    for (int i = threadIdx.x; i < nz; i += blockDim.x) s_phix[nx * ny + i] = phi_fixed(lam[i], kf.slam);
+    for (int i = threadIdx.x; i < nx * ny; i += blockDim.x) s_phix[i] = fx_pair(phi_fixed(phi[i], kf.sphi));
+    for (int i = threadIdx.x; i < nz; i += blockDim.x) s_phix[nx * ny + i] = fx_pair(phi_fixed(lam[i], kf.slam));
     __syncthreads();
     P = s_phix;
     Lm = s_phix + nx * ny;
@@ -1005,14 +1014,24 @@ __global__ void kb_green_fill(const SolveJob* __restrict__ jobs, int nx2, int ny
 }
 
 template <int SRC>
-__global__ void kb_rows_fwd(const SolveJob* __restrict__ jobs, FftPlan pl, int nrows, int ncols, int H, int nz) {
+__global__ void kb_rows_fwd(const SolveJob* __restrict__ jobs, FftPlan pl, int nrows, int ncols, int H, int nz,
+                            const PassJob* __restrict__ pass, int a, int b) {
   const SolveJob& J = jobs[blockIdx.y];
   if (SRC == 0)
     rows_fwd_body<double, 0>(J.st, J.gbuf, nullptr, J.hat, J.tw_y, pl, nrows, ncols, H, 1, nullptr, 0, nullptr,
                              nullptr, blockIdx.x, gridDim.x);
-  else
+  else {
+    PrepJob prep = {};
+    if (pass) {
+      const PassJob& Q = pass[blockIdx.y];
+      prep.ops = Q.ops; prep.a = a; prep.b = b;
+      prep.dp_p_coeff = Q.m.dp_p_coeff;
+      prep.host_factor = Q.ka.host_factor;
+      prep.out = Q.prep;
+    }
     rows_fwd_body<double, 1>(J.st, J.rho_q, J.rho, J.hat, J.tw_y, pl, nrows, ncols, H, 1, J.z_q, nz, J.lam, nullptr,
-                             blockIdx.x, gridDim.x);
+                             blockIdx.x, gridDim.x, nullptr, nullptr, true, &prep);
+  }
 }
 
 template <int MODE>
@@ -1212,7 +1231,7 @@ static bool use_conv_fused(const orbit_sc2p5d_t* c) {
 // The Green rebuild, the forward rows, the convolution and the backward
 // rows as one cooperative launch (k_conv_fused).
 template <typename T>
-static int enqueue_conv_fused(orbit_sc2p5d_t* c, orbit_bunch_t* b, cudaStream_t s, int* nl) {
+static int enqueue_conv_fused(orbit_sc2p5d_t* c, orbit_bunch_t* b, cudaStream_t s, const PrepJob& prep, int* nl) {
   ConvArgs A;
   std::memset(&A, 0, sizeof(A));
   A.st = c->d_st;
@@ -1231,11 +1250,12 @@ static int enqueue_conv_fused(orbit_sc2p5d_t* c, orbit_bunch_t* b, cudaStream_t 
   A.denom = 1.0 / (c->nx2 * c->ny2);
   A.wait_polls = c->conv_wait_polls;
   A.withhold = c->conv_withhold;
+  A.prep = prep;
   A.src = c->d_rho_q;
   A.zacc = c->d_z_q;
   A.lam_f = c->d_lam_f;  // FP32 form: float copies for its kick (null otherwise)
   A.phi_f = c->d_phi_f;
-  int items = conv_items(c);
+  const int items = conv_items(c) + (prep.out ? 1 : 0);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(items < c->conv_blocks ? items : c->conv_blocks);
   cfg.blockDim = dim3(conv_threads(c));
@@ -1257,7 +1277,7 @@ static int enqueue_conv_fused(orbit_sc2p5d_t* c, orbit_bunch_t* b, cudaStream_t 
 // Forward row transforms of the deposit (plus one block finalizing the line
 // density).
 template <typename T>
-static int enqueue_rows_fwd(orbit_sc2p5d_t* c, cudaStream_t s, int* nl) {
+static int enqueue_rows_fwd(orbit_sc2p5d_t* c, cudaStream_t s, const PrepJob& prep, int* nl) {
   typedef typename CT<T>::t C;
   C* hat = (C*)c->d_hat;
   const C* twy = (const C*)c->d_tw_y;
@@ -1266,7 +1286,7 @@ static int enqueue_rows_fwd(orbit_sc2p5d_t* c, cudaStream_t s, int* nl) {
   int blocks = (c->nx + 1) / 2 + 1;
   ORBIT_PB("fft_rows_fwd", s);
   k_rows_fwd<T, 1><<<blocks, thy, smy, s>>>(c->d_st, c->d_rho_q, c->d_rho, hat, twy, c->plan_y, c->nx, c->ny,
-                                            c->H, 1, c->d_z_q, c->nz, c->d_lam, c->d_lam_f);
+                                            c->H, 1, c->d_z_q, c->nz, c->d_lam, c->d_lam_f, prep);
   ORBIT_PE(s);
   ++*nl;
   ORBIT_LAUNCH_CHECK("sc2p5d rows");
@@ -1318,7 +1338,8 @@ static int enqueue_green(orbit_sc2p5d_t* c, cudaStream_t s, int gate, void* scra
   ORBIT_PB("green_rows", s);
   C* hat = (C*)scratch;
   k_rows_fwd<T, 0><<<(c->nx + 2) / 2, thy, smy, s>>>(c->d_st, c->d_gbuf, nullptr, hat, twy, c->plan_y,
-                                                      c->nx + 1, c->ny2, c->H, gate, nullptr, 0, nullptr, nullptr);
+                                                      c->nx + 1, c->ny2, c->H, gate, nullptr, 0, nullptr, nullptr,
+                                                      PrepJob{});
   ORBIT_PE(s);
   ORBIT_PB("green_cols", s);
   k_cols<T, 0><<<c->H, thx, smx, s>>>(c->d_st, hat, green, twx, c->plan_x, c->nx2, c->H, c->ny2, gate);
@@ -1379,7 +1400,8 @@ int batch_enqueue_green(const SolveJob* jobs, int nm, const orbit_sc2p5d_t* c, i
   kb_green_fill<<<dim3(gb, nm), 256, 0, s>>>(jobs, c->nx2, c->ny2);
   ORBIT_PE(s);
   ORBIT_PB("batch_green_rows", s);
-  kb_rows_fwd<0><<<dim3((c->nx + 2) / 2, nm), thy, smy, s>>>(jobs, c->plan_y, c->nx + 1, c->ny2, c->H, 0);
+  kb_rows_fwd<0><<<dim3((c->nx + 2) / 2, nm), thy, smy, s>>>(jobs, c->plan_y, c->nx + 1, c->ny2, c->H, 0, nullptr, 0,
+                                                                 0);
   ORBIT_PE(s);
   ORBIT_PB("batch_green_cols", s);
   kb_cols<0><<<dim3(c->H, nm), thx, smx, s>>>(jobs, c->plan_x, c->nx2, c->H, c->ny2);
@@ -1421,11 +1443,12 @@ int batch_enqueue_fft_probe(const SolveJob* jobs, int nm, const orbit_sc2p5d_t* 
 // backward rows, and the fixed-point potential for kicks that read it from
 // global memory.
 int batch_enqueue_solve(const SolveJob* jobs, int nm, const orbit_sc2p5d_t* c, int fft_wide, bool phi_fix,
-                        cudaStream_t s) {
+                        const PassJob* pass, int a, int b, cudaStream_t s) {
   int thx = batch_fft_threads(c->plan_x, fft_wide), thy = batch_fft_threads(c->plan_y, fft_wide);
   size_t smx = fft_smem<double>(c->nx2), smy = fft_smem<double>(c->ny2);
   ORBIT_PB("batch_rows_fwd", s);
-  kb_rows_fwd<1><<<dim3((c->nx + 1) / 2 + 1, nm), thy, smy, s>>>(jobs, c->plan_y, c->nx, c->ny, c->H, c->nz);
+  kb_rows_fwd<1><<<dim3((c->nx + 1) / 2 + 1, nm), thy, smy, s>>>(jobs, c->plan_y, c->nx, c->ny, c->H, c->nz,
+                                                                     pass, a, b);
   ORBIT_PE(s);
   ORBIT_PB("batch_cols_conv", s);
   kb_cols<1><<<dim3(c->H, nm), thx, smx, s>>>(jobs, c->plan_x, c->nx, c->H, c->ny2);
@@ -1503,6 +1526,7 @@ SetupArgs sc_setup_args(const orbit_sc2p5d_t* c, const DepScales& d, const orbit
   sa.ny = c->ny;
   sa.nz = c->nz;
   sa.rb = c->rb ? 1 : 0;
+  sa.mag = c->form == ORBIT_FORM_PLAIN && !c->rb;
   sa.cond = 0;
   sa.bnd = 0;
   sa.bxmin = sa.bxmax = sa.bymin = sa.bymax = 0.0;
@@ -1578,7 +1602,7 @@ static void enqueue_check_solve(orbit_sc2p5d_t* c, cudaStream_t s) {
   const size_t smx = fft_smem<T>(c->nx2), smy = fft_smem<T>(c->ny2);
   k_rows_fwd<T, 3><<<(c->nx + 1) / 2, thy, smy, s>>>(c->d_dn_st, c->d_dn_raw, nullptr, (C*)c->d_dn_hat,
                                                        (const C*)c->d_tw_y, c->plan_y, c->nx, c->ny, c->H, 1,
-                                                       nullptr, 0, nullptr, nullptr);
+                                                       nullptr, 0, nullptr, nullptr, PrepJob{});
   k_cols<T, 1><<<c->H, thx, smx, s>>>(c->d_dn_st, (C*)c->d_dn_hat, (C*)c->d_green, (const C*)c->d_tw_x, c->plan_x,
                                         c->nx, c->H, c->ny2, 1);
   k_rows_inv<T><<<(c->nx + 1) / 2, thy, smy, s>>>(c->d_dn_st, (const C*)c->d_dn_hat, (const C*)c->d_tw_y,
@@ -1587,8 +1611,10 @@ static void enqueue_check_solve(orbit_sc2p5d_t* c, cudaStream_t s) {
 }
 
 int sc_enqueue_kick(orbit_sc2p5d_t* c, orbit_bunch_t* b, double length, cudaStream_t s, bool do_extrema,
-                    bool do_kick, int* launches, double pipe_radius, const orbit_boundary* bnd) {
+                    bool do_kick, int* launches, double pipe_radius, const orbit_boundary* bnd,
+                    const PrepJob* prep_job) {
   int nl = 0;
+  const PrepJob prep = prep_job ? *prep_job : PrepJob{};
   const int n = b->n;
   const double* msz = b->has_msize ? b->d_msize : nullptr;
   const bool plain = c->form == ORBIT_FORM_PLAIN;
@@ -1693,10 +1719,10 @@ int sc_enqueue_kick(orbit_sc2p5d_t* c, orbit_bunch_t* b, double length, cudaStre
     if (rc) return rc;
   }
   if (fused) {
-    rc = plain ? enqueue_conv_fused<double>(c, b, s, &nl) : enqueue_conv_fused<float>(c, b, s, &nl);
+    rc = plain ? enqueue_conv_fused<double>(c, b, s, prep, &nl) : enqueue_conv_fused<float>(c, b, s, prep, &nl);
     if (rc) return rc;
   } else {
-    rc = plain ? enqueue_rows_fwd<double>(c, s, &nl) : enqueue_rows_fwd<float>(c, s, &nl);
+    rc = plain ? enqueue_rows_fwd<double>(c, s, prep, &nl) : enqueue_rows_fwd<float>(c, s, prep, &nl);
     if (rc) return rc;
   }
   if (c->rb) {
@@ -1853,6 +1879,7 @@ int orbit_sc2p5d_create(orbit_sc2p5d_t** out, int nx, int ny, int nz, double xy_
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking);
   A((void**)&c->d_st, sizeof(ScState));
+  A((void**)&c->d_prep, sizeof(PassPrep));
   A((void**)&c->d_rho, sizeof(double) * ng);
   A((void**)&c->d_phi, sizeof(double) * ng);
   A((void**)&c->d_lam, sizeof(double) * nz);
@@ -1917,7 +1944,7 @@ int orbit_sc2p5d_destroy(orbit_sc2p5d_t* c) {
   if (c->used) cudaEventSynchronize(c->done);
   if (c->done) cudaEventDestroy(c->done);
   if (c->aux) cudaStreamDestroy(c->aux);
-  void* ptrs[] = {c->d_st, c->d_rho_q, c->d_z_q, c->d_rho, c->d_phi, c->d_lam, c->d_lamd,
+  void* ptrs[] = {c->d_st, c->d_prep, c->d_rho_q, c->d_z_q, c->d_rho, c->d_phi, c->d_lam, c->d_lamd,
                   c->d_phi_f, c->d_lam_f, c->d_hat, c->d_green, c->d_gbuf, c->d_gscratch, c->d_tw_x, c->d_tw_y,
                   c->d_phi_fix, c->d_lam_fix, c->d_dn_parts, c->d_dn_raw, c->d_dn_hat, c->d_dn_phi,
                   c->d_dn_st};

@@ -17,7 +17,8 @@ struct ScState {
   double xy_ratio;                                        // calculator's xy_ratio (persists)
   double sxmin, sxmax, symin, symax, sdx, sdy;            // Poisson-solver grid
   double re00;                                            // Re G~[0][0] (PoissonSolverFFT2D.cc:164)
-  double scale;                                           // log(dx_solver/dx_rho) (:213)
+  double scale_arg;                                       // dx_solver/dx_rho
+  double scale;                                           // its logarithm (:213), formed beside the forward rows
   double total_m;                                         // sum of the line density (:229-233)
   double inv_qscale;                                      // macrosize per unit of the fixed-point deposit
   int green_dirty;                                        // Green spectrum must be rebuilt
@@ -39,6 +40,18 @@ struct ScState {
   // arrival counters of the fused convolution's two grid-wide barriers,
   // zeroed by every kick's set-up
   unsigned conv_bar[2];
+  // magnitudes of the bunch for the fixed-point maps of the next pass,
+  // accumulated by a lattice pass beside the extrema: largest high words of
+  // |xp|, |yp| and of |dE|, sums of the clamped exponents of x, y and of xp,
+  // yp over every thread's first particle and their number; the set-up moves
+  // them to `mag` (zero after a scan that has none)
+  unsigned acc_pmax, acc_emax, acc_n;
+  unsigned long long acc_sx, acc_sp;
+  struct {
+    unsigned pmax, emax, n;
+    unsigned long long sx, sp;
+    double xmax;  // max |x|, |y| before the grid is stretched
+  } mag;
 };
 
 // Inside test of a conducting boundary (BaseBoundary2D.cc:144-151,
@@ -69,6 +82,7 @@ struct SetupArgs {
   double inv_qscale;  // macrosize per unit of the fixed-point deposit (1 for the fp32 form)
   int nx, ny, nz;
   int rb;             // SpaceChargeCalc2p5Drb set-up: fixed ratio, solver grid never reshaped
+  int mag;            // the scan accumulates the magnitudes a fixed-point pass needs (plain form)
   int bnd;            // a conducting boundary fixes the transverse grid to its extents
   double bxmin, bxmax, bymin, bymax;
   cudaGraphConditionalHandle cond;  // inside a graph: the Green-rebuild branch of this kick (0: none)
@@ -92,6 +106,20 @@ struct FftPlan {
 
 struct orbit_boundary;
 struct orbit_denoiser;
+
+namespace orbit {
+struct DevOp;
+struct PassPrep;
+// The lattice pass that follows a kick, for the constants made beside its
+// solve (prep_pass): maps ops[a..b), dp_p per dE and the kick factor; out
+// null: none.
+struct PrepJob {
+  const DevOp* ops;
+  int a, b;
+  double dp_p_coeff, host_factor;
+  PassPrep* out;
+};
+}  // namespace orbit
 
 namespace orbit {
 // The denoiser's device error flag (tensor-core waits that gave up).
@@ -123,12 +151,13 @@ struct orbit_sc2p5d {
   double* d_lam = nullptr;                // user-visible line density (nz)
   float* d_phi_f = nullptr;               // fp32-form phi
   float* d_lam_f = nullptr;
-  long long* d_phi_fix = nullptr;         // plain form: phi, lambda as scaled 64-bit integers
+  long long* d_phi_fix = nullptr;         // plain form: phi, lambda as scaled 64-bit integers (as fx::V pairs)
   long long* d_lam_fix = nullptr;
   void* d_hat = nullptr;                  // nx2 * H complex work spectrum (T = double or float)
   void* d_green = nullptr;                // nx2 * H complex Green spectrum
   double* d_gbuf = nullptr;               // nx2 * ny2 real Green function
   void* d_gscratch = nullptr;             // nx2 * H complex: Green row spectra inside a graph
+  orbit::PassPrep* d_prep = nullptr;      // constants of the pass after the kick (prep_pass)
   void* d_tw_x = nullptr;                 // twiddles for N = nx2
   void* d_tw_y = nullptr;                 // twiddles for N = ny2
   orbit::FftPlan plan_x{}, plan_y{};
@@ -178,9 +207,11 @@ namespace orbit {
 // `do_extrema` = false when the extrema keys were already accumulated by a
 // fused pass; `do_kick` = false when the kick is deferred to the next fused
 // pass.  Returns the number of kernel launches added through *launches.
+// prep: the constants of the fixed-point pass that follows are made beside
+// the solve.
 int sc_enqueue_kick(orbit_sc2p5d_t* c, orbit_bunch_t* b, double length, cudaStream_t st,
                     bool do_extrema, bool do_kick, int* launches, double pipe_radius = 0.0,
-                    const orbit_boundary* bnd = nullptr);
+                    const orbit_boundary* bnd = nullptr, const PrepJob* prep = nullptr);
 // Cross-stream ordering of a calculator's buffers: work on stream s waits
 // for the last recorded use, then records a new one.
 cudaError_t sc_order_before(orbit_sc2p5d_t* c, cudaStream_t s);

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fixmap.cuh"
 #include "softf64.cuh"
 #include "sc2p5d.cuh"
 
@@ -30,133 +31,205 @@ struct ExtAcc {
   }
 };
 
-// Block-wide reduction, then one atomic per key per block.
-__device__ __forceinline__ void ext_block_commit(ExtAcc& a, ScState* st, unsigned* status) {
-  __shared__ unsigned long long s_k[32][6];
-  __shared__ int s_bad;
-  if (threadIdx.x == 0) s_bad = 0;
-  for (int c = 0; c < 3; ++c) {
-    for (int off = 16; off > 0; off >>= 1) {
-      unsigned long long o1 = __shfl_xor_sync(0xffffffffu, a.mn[c], off);
-      unsigned long long o2 = __shfl_xor_sync(0xffffffffu, a.mx[c], off);
-      a.mn[c] = o1 < a.mn[c] ? o1 : a.mn[c];
-      a.mx[c] = o2 > a.mx[c] ? o2 : a.mx[c];
-    }
+// Magnitudes of a bunch (ScState::mag): largest high words of |xp|, |yp| and
+// |dE|, and sums of the exponents of x, y and xp, yp clamped to 2^-60..2^60
+// (integer maxima and sums: the same on every run).
+struct MagAcc {
+  unsigned pm, em, sx, sp, n;
+  __device__ __forceinline__ void init() { pm = em = sx = sp = n = 0u; }
+  static __device__ __forceinline__ unsigned hi(double v) {
+    return (unsigned)__double2hiint(v) & 0x7fffffffu;
   }
-  __syncthreads();
-  if (a.bad) s_bad = 1;
-  int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  static __device__ __forceinline__ unsigned ex(double v) {
+    const unsigned h = hi(v) >> 20;
+    return h < 963u ? 963u : (h > 1083u ? 1083u : h);
+  }
+  __device__ __forceinline__ void bound(double xp, double yp) { pm = max(pm, max(hi(xp), hi(yp))); }
+  __device__ __forceinline__ void sample(double x, double xp, double y, double yp) {
+    sx += ex(x) + ex(y);
+    sp += ex(xp) + ex(yp);
+    ++n;
+  }
+  __device__ __forceinline__ void add(double x, double xp, double y, double yp, double dE) {
+    bound(xp, yp);
+    em = max(em, hi(dE));
+    sample(x, xp, y, yp);
+  }
+};
+
+// Block-wide reduction, one atomic per quantity per block.
+__device__ __forceinline__ void mag_block_commit(const MagAcc& a, ScState* st) {
+  __shared__ unsigned s_m[5][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu;
+  const unsigned v[5] = {__reduce_max_sync(full, a.pm), __reduce_max_sync(full, a.em), __reduce_add_sync(full, a.sx),
+                         __reduce_add_sync(full, a.sp), __reduce_add_sync(full, a.n)};
   if (lane == 0)
-    for (int c = 0; c < 3; ++c) { s_k[w][2 * c] = a.mn[c]; s_k[w][2 * c + 1] = a.mx[c]; }
+    for (int k = 0; k < 5; ++k) s_m[k][w] = v[k];
   __syncthreads();
-  if (threadIdx.x < 6) {
-    int nw = (blockDim.x + 31) >> 5;
-    unsigned long long v = s_k[0][threadIdx.x];
-    bool is_min = (threadIdx.x & 1) == 0;
-    for (int q = 1; q < nw; ++q) {
-      unsigned long long u = s_k[q][threadIdx.x];
-      v = is_min ? (u < v ? u : v) : (u > v ? u : v);
+  if (w < 5) {  // one warp per quantity (a block has at least that many, or its warps take turns)
+    const int nw = (blockDim.x + 31) >> 5;
+    for (int k = w; k < 5; k += nw) {
+      const unsigned u = lane < nw ? s_m[k][lane] : 0u;
+      const unsigned r = k < 2 ? __reduce_max_sync(full, u) : __reduce_add_sync(full, u);
+      if (lane == 0) {
+        if (k < 2) atomicMax(k == 0 ? &st->acc_pmax : &st->acc_emax, r);
+        else if (k < 4) atomicAdd(k == 2 ? &st->acc_sx : &st->acc_sp, (unsigned long long)r);
+        else atomicAdd(&st->acc_n, r);
+      }
     }
-    if (is_min) atomicMin(&st->key[threadIdx.x], v);
-    else atomicMax(&st->key[threadIdx.x], v);
   }
-  if (threadIdx.x == 0 && s_bad) atomicOr(status, (unsigned)ST_NAN);
+}
+
+// Smallest 64-bit key of a warp, from two 32-bit reductions.
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+  const unsigned h = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32));
+  const unsigned l = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32) == h ? (unsigned)k : ~0u);
+  return ((unsigned long long)h << 32) | l;
+}
+
+// Block-wide reduction, then one atomic per key per block (a maximum is the
+// complement's minimum).
+__device__ __forceinline__ void ext_block_commit(ExtAcc& a, ScState* st, unsigned* status) {
+  __shared__ unsigned long long s_k[6][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    const unsigned long long lo = c == 0 ? a.mn[0] : c == 1 ? a.mn[1] : a.mn[2];
+    const unsigned long long hi = c == 0 ? a.mx[0] : c == 1 ? a.mx[1] : a.mx[2];
+    const unsigned long long v0 = warp_min_key(lo), v1 = warp_min_key(~hi);
+    if (lane == 0) {
+      s_k[2 * c][w] = v0;
+      s_k[2 * c + 1][w] = v1;
+    }
+  }
+  const int bad = __syncthreads_or(a.bad);
+#pragma unroll 1
+  for (int k = w; k < 6; k += nw) {
+    const unsigned long long v = warp_min_key(lane < nw ? s_k[k][lane] : ~0ull);
+    if (lane == 0) {
+      if (k & 1) atomicMax(&st->key[k], ~v);
+      else atomicMin(&st->key[k], v);
+    }
+  }
+  if (threadIdx.x == 0 && bad) atomicOr(status, (unsigned)ST_NAN);
 }
 
 // ---------------------------------------------------------------------
 // Grid set-up of bunchAnalysis (SpaceChargeCalc2p5D.cc:126-216), run by
-// one thread of the last block of the kernel that scanned the extrema.
+// one warp of the last block of the kernel that scanned the extrema.
 // ---------------------------------------------------------------------
 // Explicitly rounded operations (no contraction), so that the grid limits
 // and the persistent xy_ratio evolve exactly as the reference's.  The keys
 // and the status word were written by atomics of other blocks: they are
 // read from L2.
-static __device__ __noinline__ void sc_setup_scalar(ScState* st, unsigned* status, SetupArgs sa) {
+//
+// The set-up is a chain of divisions on the critical path of every kick.  They
+// run on the integer pipes (sf::div, correctly rounded as the instruction);
+// every lane follows the same steps, and divisions that do not hang on one
+// another go to different lanes of one division (four in a row instead of
+// fourteen); halves are products by 0.5 (the same value), and the logarithm of
+// the solver's scale is left to a block beside the forward rows.
+static __device__ __noinline__ void sc_setup_warp(ScState* st, unsigned* status, const SetupArgs& sa) {
+  const int lane = threadIdx.x & 31;
   unsigned long long key[6];
   for (int c = 0; c < 6; ++c) key[c] = __ldcg(&st->key[c]);
+  const double xy0 = st->xy_ratio, sxmin = st->sxmin, sxmax = st->sxmax, symin = st->symin, symax = st->symax;
+  const double sdx0 = st->sdx;
+  const unsigned stat = __ldcg(status);
   double xMin = dkey_inv(key[0]), xMax = dkey_inv(key[1]);
   double yMin = dkey_inv(key[2]), yMax = dkey_inv(key[3]);
   double zMin = dkey_inv(key[4]), zMax = dkey_inv(key[5]);
-  for (int c = 0; c < 3; ++c) { st->key[2 * c] = ~0ull; st->key[2 * c + 1] = 0ull; }
-  st->conv_bar[0] = 0u;
-  st->conv_bar[1] = 0u;
+  __syncwarp();
+  if (lane == 0) {
+    for (int c = 0; c < 3; ++c) { st->key[2 * c] = ~0ull; st->key[2 * c + 1] = 0ull; }
+    st->mag.pmax = __ldcg(&st->acc_pmax);
+    st->mag.emax = __ldcg(&st->acc_emax);
+    st->mag.n = __ldcg(&st->acc_n);
+    st->mag.sx = __ldcg(&st->acc_sx);
+    st->mag.sp = __ldcg(&st->acc_sp);
+    st->mag.xmax = fmax(fmax(fabs(xMin), fabs(xMax)), fmax(fabs(yMin), fabs(yMax)));
+    st->acc_pmax = st->acc_emax = st->acc_n = 0u;
+    st->acc_sx = st->acc_sp = 0ull;
+    st->conv_bar[0] = 0u;
+    st->conv_bar[1] = 0u;
+  }
   if (sa.bnd) {
     // a boundary fixes the transverse grid to its extents; only z comes
     // from the bunch (SpaceChargeCalc2p5D.cc:174-196)
     xMin = sa.bxmin; xMax = sa.bxmax; yMin = sa.bymin; yMax = sa.bymax;
   }
-  int skip = 0;
-  if (__ldcg(status) & ST_NAN) {
+  if (stat & ST_NAN) {
     // a non-finite coordinate was met by the extrema scan: no kick
-    skip = 1;
-  } else if (!(xMin < xMax) || !(yMin < yMax) || !(zMin < zMax)) {  // :131 (also catches an empty scan)
-    skip = 1;
-    atomicOr(status, (unsigned)ST_EXTENT);
-  } else {
-    double xy = st->xy_ratio;
-    double ratio_beam = __ddiv_rn(__dsub_rn(xMax, xMin), __dsub_rn(yMax, yMin));
-    int set_solver = 0;
-    if (sa.bnd) {
-      xy = ratio_beam;  // :180
-    } else if (sa.rb) {
-      // SpaceChargeCalc2p5Drb::bunchAnalysis (SpaceChargeCalc2p5Drb.cc:188-203):
-      // always stretched to the calculator's own ratio, which never changes
-      double width, center;
-      if (ratio_beam > xy) {
-        center = __ddiv_rn(__dadd_rn(yMax, yMin), 2.0);
-        width = __ddiv_rn(__dmul_rn(__dsub_rn(yMax, yMin), __ddiv_rn(ratio_beam, xy)), 2.0);
-        yMin = __dsub_rn(center, width);
-        yMax = __dadd_rn(center, width);
-      } else {
-        center = __ddiv_rn(__dadd_rn(xMax, xMin), 2.0);
-        width = __ddiv_rn(__ddiv_rn(__dsub_rn(xMax, xMin), __ddiv_rn(ratio_beam, xy)), 2.0);
-        xMin = __dsub_rn(center, width);
-        xMax = __dadd_rn(center, width);
-      }
-    } else if (fabs(__dsub_rn(ratio_beam, xy)) < __dmul_rn(0.25, xy)) {  // :152-168
-      double width, center;
-      if (ratio_beam > xy) {
-        center = __ddiv_rn(__dadd_rn(yMax, yMin), 2.0);
-        width = __ddiv_rn(__dmul_rn(__dsub_rn(yMax, yMin), __ddiv_rn(ratio_beam, xy)), 2.0);
-        yMin = __dsub_rn(center, width);
-        yMax = __dadd_rn(center, width);
-      } else {
-        center = __ddiv_rn(__dadd_rn(xMax, xMin), 2.0);
-        width = __ddiv_rn(__ddiv_rn(__dsub_rn(xMax, xMin), __ddiv_rn(ratio_beam, xy)), 2.0);
-        xMin = __dsub_rn(center, width);
-        xMax = __dadd_rn(center, width);
-      }
-      xy = __ddiv_rn(__dsub_rn(xMax, xMin), __dsub_rn(yMax, yMin));
-    } else {  // :169-173
-      xy = ratio_beam;
-      set_solver = 1;
-    }
-    // Grid2D::setGridX/Y (Grid2D.cc:422-433), Grid1D::setGridZ (Grid1D.cc:89-94)
-    double dx = __ddiv_rn(__dsub_rn(xMax, xMin), (double)(sa.nx - 1));
-    double dy = __ddiv_rn(__dsub_rn(yMax, yMin), (double)(sa.ny - 1));
-    double dz = __ddiv_rn(__dsub_rn(zMax, zMin), (double)sa.nz);
-    st->xmin = xMin; st->xmax = xMax; st->ymin = yMin; st->ymax = yMax;
-    st->dx = dx; st->dy = dy; st->inv_dx = __drcp_rn(dx); st->inv_dy = __drcp_rn(dy);
-    st->zmin = zMin; st->zmax = zMax; st->dz = dz; st->inv_dz = __drcp_rn(dz);
-    if (!sa.rb) st->xy_ratio = xy;
-    // solver-shape check (SpaceChargeCalc2p5D.cc:208-216); the 2.5Drb
-    // calculator keeps its solver grid
-    if (!set_solver && !sa.rb) {
-      double sr = __ddiv_rn(__dsub_rn(st->sxmax, st->sxmin), __dsub_rn(st->symax, st->symin));
-      if (fabs(__dsub_rn(sr, xy)) > 0.00000001) set_solver = 1;
-    }
-    if (set_solver) {  // PoissonSolverFFT2D::setGridXY (PoissonSolverFFT2D.cc:103-111)
-      st->sxmin = xMin; st->sxmax = xMax; st->symin = yMin; st->symax = yMax;
-      st->sdx = dx; st->sdy = dy;
-      st->green_dirty = 1;
-    }
-    st->scale = log(__ddiv_rn(st->sdx, dx));  // PoissonSolverFFT2D.cc:213
-    st->inv_qscale = sa.inv_qscale;
-    st->phi_absmax = 0ull;
-    st->lam_absmax = 0ull;
-    if (sa.cond) cudaGraphSetConditional(sa.cond, st->green_dirty ? 1u : 0u);
+    if (lane == 0) st->skip = 1;
+    return;
   }
-  st->skip = skip;
+  if (!(xMin < xMax) || !(yMin < yMax) || !(zMin < zMax)) {  // :131 (also catches an empty scan)
+    if (lane == 0) {
+      st->skip = 1;
+      atomicOr(status, (unsigned)ST_EXTENT);
+    }
+    return;
+  }
+  // lane q divides num by den; the quotients of lanes 0..3
+  auto div4 = [](double n0, double d0, double n1, double d1, double n2, double d2, double n3, double d3, double q[4]) {
+    const int l = threadIdx.x & 3;
+    const double v = sf::div(l == 0 ? n0 : l == 1 ? n1 : l == 2 ? n2 : n3, l == 0 ? d0 : l == 1 ? d1 : l == 2 ? d2 : d3);
+    for (int k = 0; k < 4; ++k) q[k] = __shfl_sync(0xffffffffu, v, k);
+  };
+  double q[4];
+  double xy = xy0;
+  div4(__dsub_rn(xMax, xMin), __dsub_rn(yMax, yMin), __dsub_rn(sxmax, sxmin), __dsub_rn(symax, symin),
+       __dsub_rn(zMax, zMin), (double)sa.nz, 1.0, 1.0, q);
+  const double ratio_beam = q[0], sr = q[1], dz = q[2];
+  int set_solver = 0;
+  if (sa.bnd) {
+    xy = ratio_beam;  // :180
+  } else if (sa.rb || fabs(__dsub_rn(ratio_beam, xy)) < __dmul_rn(0.25, xy)) {
+    // :152-168; SpaceChargeCalc2p5Drb::bunchAnalysis (SpaceChargeCalc2p5Drb.cc:188-203)
+    // always stretches to the calculator's own ratio, which never changes
+    const double rr = sf::div(ratio_beam, xy);
+    double width, center;
+    if (ratio_beam > xy) {
+      center = __dmul_rn(__dadd_rn(yMax, yMin), 0.5);
+      width = __dmul_rn(__dmul_rn(__dsub_rn(yMax, yMin), rr), 0.5);
+      yMin = __dsub_rn(center, width);
+      yMax = __dadd_rn(center, width);
+    } else {
+      center = __dmul_rn(__dadd_rn(xMax, xMin), 0.5);
+      width = __dmul_rn(sf::div(__dsub_rn(xMax, xMin), rr), 0.5);
+      xMin = __dsub_rn(center, width);
+      xMax = __dadd_rn(center, width);
+    }
+  } else {  // :169-173
+    xy = ratio_beam;
+    set_solver = 1;
+  }
+  // Grid2D::setGridX/Y (Grid2D.cc:422-433), Grid1D::setGridZ (Grid1D.cc:89-94)
+  div4(__dsub_rn(xMax, xMin), (double)(sa.nx - 1), __dsub_rn(yMax, yMin), (double)(sa.ny - 1),
+       __dsub_rn(xMax, xMin), __dsub_rn(yMax, yMin), 1.0, dz, q);
+  const double dx = q[0], dy = q[1], inv_dz = q[3];
+  if (!sa.bnd && !sa.rb && !set_solver) xy = q[2];
+  // solver-shape check (SpaceChargeCalc2p5D.cc:208-216); the 2.5Drb
+  // calculator keeps its solver grid
+  if (!set_solver && !sa.rb && fabs(__dsub_rn(sr, xy)) > 0.00000001) set_solver = 1;
+  div4(1.0, dx, 1.0, dy, set_solver ? dx : sdx0, dx, 1.0, 1.0, q);
+  if (lane != 0) return;
+  st->xmin = xMin; st->xmax = xMax; st->ymin = yMin; st->ymax = yMax;
+  st->dx = dx; st->dy = dy; st->inv_dx = q[0]; st->inv_dy = q[1];
+  st->zmin = zMin; st->zmax = zMax; st->dz = dz; st->inv_dz = inv_dz;
+  if (!sa.rb) st->xy_ratio = xy;
+  if (set_solver) {  // PoissonSolverFFT2D::setGridXY (PoissonSolverFFT2D.cc:103-111)
+    st->sxmin = xMin; st->sxmax = xMax; st->symin = yMin; st->symax = yMax;
+    st->sdx = dx; st->sdy = dy;
+    st->green_dirty = 1;
+  }
+  st->scale_arg = q[2];  // its logarithm: PoissonSolverFFT2D.cc:213
+  st->inv_qscale = sa.inv_qscale;
+  st->phi_absmax = 0ull;
+  st->lam_absmax = 0ull;
+  if (sa.cond) cudaGraphSetConditional(sa.cond, (set_solver || st->green_dirty) ? 1u : 0u);
+  st->skip = 0;
 }
 
 // True in exactly one of the nblk blocks that share `counter` (all blocks
@@ -179,12 +252,33 @@ __device__ __forceinline__ bool last_block_done(unsigned* counter, unsigned nblk
   return s_last != 0;
 }
 
+// Waits until *cnt reaches n, for at most `polls` polls; a wait that runs out
+// sets ST_SYNC and returns 0.  One thread; what the others wrote before they
+// arrived is visible after it.
+__device__ __forceinline__ int counter_wait(unsigned* cnt, unsigned n, long long polls, unsigned* status) {
+  int ok = 1;
+  long long i = 0;
+  for (;;) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
+    if (v >= n) break;
+    if (++i > polls) {
+      ok = 0;
+      break;
+    }
+    __nanosleep(32);
+  }
+  if (!ok) atomicOr(status, (unsigned)ST_SYNC);
+  __threadfence();
+  return ok;
+}
+
 // Extrema commit followed, in the last of the nblk blocks scanning this
 // bunch, by the grid set-up.
 __device__ __forceinline__ void ext_commit_and_setup(ExtAcc& a, ScState* st, unsigned* status,
                                                      const SetupArgs& sa, unsigned nblk) {
   ext_block_commit(a, st, status);
-  if (last_block_done(&st->ext_count, nblk) && threadIdx.x == 0) sc_setup_scalar(st, status, sa);
+  if (last_block_done(&st->ext_count, nblk) && threadIdx.x < 32) sc_setup_warp(st, status, sa);
 }
 
 // ---------------------------------------------------------------------
@@ -283,7 +377,8 @@ __device__ __forceinline__ void load_kick_const(KickConst& k, const ScState* st,
   k.xmin = st->xmin; k.ymin = st->ymin; k.inv_dx = st->inv_dx; k.inv_dy = st->inv_dy;
   k.zmin = st->zmin; k.zmax = st->zmax; k.inv_dz = st->inv_dz;
   // factor = 2 L r_c/(beta^2 gamma^3) / (z_step * totalMacrosize)  (:96-100)
-  k.fac = host_factor / (st->dz * st->total_m);
+  // (the sum may come from another block of the same launch: from L2)
+  k.fac = sf::div(host_factor, __dmul_rn(st->dz, __ldcg(&st->total_m)));
   k.nx = nx; k.ny = ny; k.nz = nz;
   k.skip = st->skip;
   if (!f32) return;
@@ -374,7 +469,6 @@ __device__ __forceinline__ void kick_plain(const KickConst& k, const double* __r
   yp += gy * k.inv_dy * lf;
 }
 
-// FP32 form: gradient and line density in FP32, accumulation into FP64.
 __device__ __forceinline__ void kick_fp32(const KickConst& k, const float* __restrict__ phi,
                                           const float* __restrict__ lam, double x, double y, double z,
                                           double& xp, double& yp) {
@@ -602,18 +696,12 @@ __device__ __forceinline__ bool tsc_fixed(double v, int n, int F, int& ind, long
   return true;
 }
 
-// 9-point weights Wm, W0, Wp (Q58) and derivative weights (Q58).
+// 9-point weights Wm, W0, Wp (Q58).
 __device__ __forceinline__ void tsc_w_fixed(long long f, long long w[3]) {
   w[0] = sq_q58(f - (1ll << 55)) >> 1;
   w[1] = (3ll << 56) - sq_q58(f);
   w[2] = sq_q58(f + (1ll << 55)) >> 1;
 }
-__device__ __forceinline__ void tsc_dw_fixed(long long f, long long dw[3]) {
-  dw[0] = (f - (1ll << 55)) << 2;  // f - 1/2
-  dw[1] = -(f << 3);               // -2 f
-  dw[2] = (f + (1ll << 55)) << 2;  // f + 1/2
-}
-
 // Grid1D index on u = (z - zmin)/dz + 0.5 (nz > 1): floor semantics with
 // periodic neighbours reproduce every wrap rule of Grid1D::getIndAndWZ;
 // wp (weight of ip) in Q56.
@@ -724,10 +812,10 @@ __device__ __forceinline__ void load_kick_fix(KickFix& k, const ScState* st, dou
   k.az = st->inv_dz; k.cz = 0.5 - st->zmin * st->inv_dz;
   k.kzmin = dkey(st->zmin); k.kzmax = dkey(st->zmax);
   k.sphi = scale_bits(st->phi_absmax);
-  k.slam = scale_bits(st->lam_absmax);
-  k.gxs = ldexp(st->inv_dx, 5 - k.sphi);
-  k.gys = ldexp(st->inv_dy, 5 - k.sphi);
-  k.lfs = ldexp(-fac, 2 - k.slam);
+  k.slam = scale_bits(__ldcg(&st->lam_absmax));
+  k.gxs = sf::pow2mul(st->inv_dx, 5 - k.sphi);
+  k.gys = sf::pow2mul(st->inv_dy, 5 - k.sphi);
+  k.lfs = sf::pow2mul(-fac, 2 - k.slam);
   k.nx = nx; k.ny = ny; k.nz = nz;
   k.Fx = fix_bits(nx); k.Fy = fix_bits(ny); k.Fz = fix_bits(nz);
   k.skip = st->skip;
@@ -757,41 +845,76 @@ __device__ __forceinline__ long long phi_fixed(double v, int s) {
   return fix_of(v, s, r) ? r : 0;
 }
 
-// Returns false when the particle needs the FP64 path.
-__device__ __forceinline__ bool kick_fixed(const KickFix& k, const long long* __restrict__ P,
-                                           const long long* __restrict__ Lm, double x, double y, double z,
-                                           double& xp, double& yp) {
-  int ix, iy;
-  long long fx, fy;
-  if (!tsc_fixed(fma(x, k.ax, k.cx), k.nx, k.Fx, ix, fx)) return false;
-  if (!tsc_fixed(fma(y, k.ay, k.cy), k.ny, k.Fy, iy, fy)) return false;
-  long long lv = 0;
-  unsigned long long kz = dkey(z);
+// A fixed-point grid value as the fx::V pair the kick multiplies (high word
+// above, signed low word below).
+__device__ __forceinline__ long long fx_pair(long long v) {
+  const fx::V p = fx::sp(v);
+  return (long long)(((unsigned long long)(unsigned)p.h << 32) | (unsigned)p.l);
+}
+__device__ __forceinline__ fx::V fx_of_pair(long long v) {
+  fx::V p;
+  p.l = (int)(unsigned)v;
+  p.h = (int)(v >> 32);
+  return p;
+}
+
+// Gradient of the fixed-point potential (Grid2D::calcGradient) at cell (ix,
+// iy) and fractions fx, fy (Q62, |f| <= 1.25): gx, gy in Q(sphi-5) cells.
+// The weights come from one square per axis, each row's two sums and the two
+// column sums are rounded once (fx::mul3): about 90 instructions for the 24
+// products against ~400 as separate 64-bit high products.
+__device__ __forceinline__ void grad_fixed(const long long* __restrict__ P, int ny, int ix, int iy, long long fx_,
+                                           long long fy_, long long& gx, long long& gy) {
+  const fx::V fx1 = fx::sp(fx_), fy1 = fx::sp(fy_);
+  const long long x2 = fx::mul(fx1, fx1) << 2, y2 = fx::mul(fy1, fy1) << 2;  // f^2, Q62
+  const long long e8 = 1ll << 59, half = 1ll << 60;
+  // W = (f -+ 1/2)^2 / 2, 3/4 - f^2 (Q62); dW = f -+ 1/2, -2 f (Q61)
+  const fx::V wxm = fx::sp((x2 >> 1) - (fx_ >> 1) + e8), wx0 = fx::sp((3ll << 60) - x2), wxp = fx::sp((x2 >> 1) + (fx_ >> 1) + e8);
+  const fx::V wym = fx::sp((y2 >> 1) - (fy_ >> 1) + e8), wy0 = fx::sp((3ll << 60) - y2), wyp = fx::sp((y2 >> 1) + (fy_ >> 1) + e8);
+  const fx::V dxm = fx::sp((fx_ >> 1) - half), dx0 = fx::sp(-fx_), dxp = fx::sp((fx_ >> 1) + half);
+  const fx::V dym = fx::sp((fy_ >> 1) - half), dy0 = fx::sp(-fy_), dyp = fx::sp((fy_ >> 1) + half);
+  fx::V s[3], t[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const long long* r = P + (ix - 1 + i) * ny + (iy - 1);
+    const fx::V a0 = fx_of_pair(r[0]), a1 = fx_of_pair(r[1]), a2 = fx_of_pair(r[2]);
+    s[i] = fx::sp(fx::mul3(wym, a0, wy0, a1, wyp, a2));  // Q(sphi-2)
+    t[i] = fx::sp(fx::mul3(dym, a0, dy0, a1, dyp, a2));  // Q(sphi-3)
+  }
+  gx = fx::mul3(dxm, s[0], dx0, s[1], dxp, s[2]);  // Q(sphi-5)
+  gy = fx::mul3(wxm, t[0], wx0, t[1], wxp, t[2]);  // Q(sphi-5)
+}
+
+// Line density at z in Q(slam-2) (Grid1D::getValue); false when the particle
+// needs the FP64 path.
+__device__ __forceinline__ bool lam_fixed(const KickFix& k, const long long* __restrict__ Lm, double z,
+                                          long long& lv) {
+  lv = 0;
+  const unsigned long long kz = dkey(z);
   if (kz >= k.kzmin && kz <= k.kzmax) {
     if (k.nz > 1) {
       int i0, ip;
       long long wp;
       if (!g1_fixed(fma(z, k.az, k.cz), k.nz, k.Fz, i0, ip, wp)) return false;
-      lv = __mul64hi(((1ll << 56) - wp) << 6, Lm[i0]) + __mul64hi(wp << 6, Lm[ip]);  // Q(slam-2)
+      wp <<= 6;
+      lv = fx::mul2(fx::sp((1ll << 62) - wp), fx_of_pair(Lm[i0]), fx::sp(wp), fx_of_pair(Lm[ip]));
     } else {
-      lv = Lm[0] >> 2;
+      lv = fx::join(fx_of_pair(Lm[0])) >> 2;
     }
   }
-  long long wx[3], wy[3], dwx[3], dwy[3];
-  tsc_w_fixed(fx, wx);
-  tsc_w_fixed(fy, wy);
-  tsc_dw_fixed(fx, dwx);
-  tsc_dw_fixed(fy, dwy);
-  long long gx = 0, gy = 0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const long long* r = P + (ix - 1 + i) * k.ny + (iy - 1);
-    long long a0 = r[0], a1 = r[1], a2 = r[2];
-    long long s = __mul64hi(wy[0] << 4, a0) + __mul64hi(wy[1] << 4, a1) + __mul64hi(wy[2] << 4, a2);     // Q(sphi-2)
-    long long t = __mul64hi(dwy[0] << 3, a0) + __mul64hi(dwy[1] << 3, a1) + __mul64hi(dwy[2] << 3, a2);  // Q(sphi-3)
-    gx += __mul64hi(dwx[i] << 3, s);  // Q(sphi-5)
-    gy += __mul64hi(wx[i] << 4, t);   // Q(sphi-5)
-  }
+  return true;
+}
+
+// Returns false when the particle needs the FP64 path.
+__device__ __forceinline__ bool kick_fixed(const KickFix& k, const long long* __restrict__ P,
+                                           const long long* __restrict__ Lm, double x, double y, double z,
+                                           double& xp, double& yp) {
+  int ix, iy;
+  long long fx, fy, lv, gx, gy;
+  if (!tsc_fixed(fma(x, k.ax, k.cx), k.nx, k.Fx, ix, fx)) return false;
+  if (!tsc_fixed(fma(y, k.ay, k.cy), k.ny, k.Fy, iy, fy)) return false;
+  if (!lam_fixed(k, Lm, z, lv)) return false;
+  grad_fixed(P, k.ny, ix, iy, fx << 6, fy << 6, gx, gy);
   const double lf = dmul<(ORBIT_SOFT_MUL >> 4) & 1>((double)lv, k.lfs);  // -lambda(z) * factor
   xp = fma((double)gx, dmul<(ORBIT_SOFT_MUL >> 4) & 1>(k.gxs, lf), xp);
   yp = fma((double)gy, dmul<(ORBIT_SOFT_MUL >> 4) & 1>(k.gys, lf), yp);

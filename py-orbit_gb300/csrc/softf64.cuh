@@ -16,6 +16,7 @@
 // them against the host's IEEE arithmetic.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -269,6 +270,77 @@ static __host__ __device__ __noinline__
 #else
 inline
 #endif
+double hw_div(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __ddiv_rn(a, b);
+#else
+  return a / b;
+#endif
+}
+
+// a / b, correctly rounded, by Newton's iteration on the integer pipes.  One
+// FP64 division is a chain of dependent FP64 operations, about 1700 clocks on
+// GB300; this chain is about 400.  With the significands as fractions m in
+// [1/2, 1) of 2^64, r ~ 1/m_b starts from the float reciprocal (error below
+// 2^-22), one step squares that to 2^-43, a second to below 2^-59; the
+// quotient m_a r, in [1/2, 2), is then off by less than four units of 2^-61.
+// Its 56-bit truncation is corrected by the exact remainder m_a 2^k - q m_b,
+// which also decides the rounding.  Zero, subnormal and non-finite operands
+// and results outside the normal range take the hardware instruction.  Out of
+// line: it runs a few times in code that each kernel enters once, where the
+// instructions' way from L2 is most of the time.
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__
+#else
+inline
+#endif
+double div(double a, double b) {
+  const uint64_t A = bits(a), B = bits(b);
+  const int ea = (int)(A >> 52) & 0x7FF, eb = (int)(B >> 52) & 0x7FF;
+  const int e = ea - eb + 1023;
+  if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)(e - 2) >= 2043u) return hw_div(a, b);
+  const uint64_t frac = (1ull << 52) - 1;
+  const uint64_t ma = (A & frac) | (1ull << 52), mb = (B & frac) | (1ull << 52);
+  const uint64_t d = mb << 11;  // m_b 2^64, top bit set
+  // r = 1/m_b in units of 2^-62, in (2^62, 2^63]
+#ifdef __CUDA_ARCH__
+  const float f = __fdividef(1.0f, (float)(uint32_t)(d >> 40));
+#else
+  const float f = 1.0f / (float)(uint32_t)(d >> 40);
+#endif
+  // f = 2^-24 / (top 24 bits of m_b) up to rounding: r0 = f 2^(24 + 62)
+  uint64_t r = (uint64_t)(f * 9007199254740992.0f) << 33;  // f 2^53, then 2^33
+  if (r > (1ull << 63)) r = 1ull << 63;
+  // r <- r (2 - m_b r): t = m_b r in units of 2^-62, near 2^62
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int k = 0; k < 2; ++k) {
+    const int64_t t = (int64_t)(1ull << 62) - (int64_t)mulhi64(d, r);  // 1 - m_b r, small
+    const uint64_t ta = (uint64_t)(t < 0 ? -t : t);
+    const uint64_t c = mulhi64(r, ta << 2);
+    r = t < 0 ? r - c : r + c;
+  }
+  // q = m_a / m_b in units of 2^-55 (m_a < m_b: one more bit)
+  const int s = ma < mb ? 1 : 0;
+  uint64_t q = mulhi64(ma << 11, r) >> (7 - s);  // m_a r 2^62 -> 2^(55 + s)
+  // remainder m_a 2^(55 + s) - q m_b (mod 2^64: it is small)
+  int64_t rem = (int64_t)((ma << (55 + s)) - q * mb);
+  while (rem < 0) { rem += (int64_t)mb; --q; }
+  while (rem >= (int64_t)mb) { rem -= (int64_t)mb; ++q; }
+  // 56 bits of quotient (top at bit 55), the remainder sticky
+  const uint64_t m0 = q >> 3;
+  const uint64_t rb = (q >> 2) & 1ull;
+  const bool sticky = rem != 0 || (q & 3ull) != 0;
+  const uint64_t m = m0 + (rb & ((uint64_t)sticky | (m0 & 1ull)));
+  return from_bits((((uint64_t)(e - s - 1) << 52) + m) | ((A ^ B) & 0x8000000000000000ull));
+}
+
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__
+#else
+inline
+#endif
 float hw_d2f(double x) {
 #ifdef __CUDA_ARCH__
   return __double2float_rn(x);
@@ -342,6 +414,14 @@ SF_HD double scale2(double x, int k) {
   const uint64_t X = bits(x);
   const int e = (int)(X >> 52) & 0x7FF;
   if ((unsigned)(e + k - 1) >= 2046u || e == 0 || e == 2047) return hw_mul(x, k > 0 ? 2.0 : 0.5);
+  return from_bits(X + ((uint64_t)(int64_t)k << 52));
+}
+
+// x 2^k: an exponent change where x and the result are normal, else ldexp.
+SF_HD double pow2mul(double x, int k) {
+  const uint64_t X = bits(x);
+  const int e = (int)(X >> 52) & 0x7FF;
+  if ((unsigned)(e - 1) >= 2046u || (unsigned)(e + k - 1) >= 2046u) return ldexp(x, k);
   return from_bits(X + ((uint64_t)(int64_t)k << 52));
 }
 

@@ -11,14 +11,10 @@
 #pragma once
 
 #include "common.cuh"
+#include "fixmap.cuh"
 #include "softf64.cuh"
 
 namespace orbit {
-
-struct DevOp {
-  int code, i0, i1, i2;
-  double c[12];
-};
 
 struct MapCtx {
   double dp_p_coeff;  // 1/(p*beta)   (e.g. teapotbase.cc:168)
