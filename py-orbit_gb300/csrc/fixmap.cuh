@@ -105,6 +105,33 @@ FX_HD int64_t mul2s(V a, V b, V c, V d, int64_t base = 0) {
   return mad(-c.h, d.h, mad(a.h, b.h, top(mids(c, d, mid(a, b, kRnd)), base)));
 }
 
+// base + floor(a b / 2^64), exactly: the sums floor at 2^32 and at 2^64 nest.
+// |a| < 1.6 2^62 and |b| <= 2^61, or both up to 2^62.
+FX_HD int64_t mul_floor(V a, V b, int64_t base = 0) {
+  return mad(a.h, b.h, top(mad(a.l, b.h, mad(a.h, b.l, mad(a.l, b.l, 0) >> 32)), base));
+}
+
+// The same for 0 <= base < 2^28 and products below 2^123: added at 2^32, a
+// carry less.
+FX_HD int64_t mul_floor_r(V a, V b, int base) {
+  const int64_t ll = mad(a.l, b.l, 0);
+  const int64_t t = (int64_t)(((uint64_t)(uint32_t)((int)(ll >> 63) + base) << 32) | (uint32_t)(ll >> 32));
+  return mad(a.h, b.h, mad(a.l, b.h, mad(a.h, b.l, t)) >> 32);
+}
+
+// The 9-point weights of f (Q61, a multiple of 32: Q56 shifted), as
+// floor((f - 1/2)^2 / 2) etc. in Q58 times 2^k, k >= 1.  One square: (f -+ 1/2)^2
+// = f^2 -+ f + 1/4, whose last two terms are whole units, so the floors are the
+// separate squares'.
+FX_HD void tsc_weights_q58(int64_t f61, int k, V w[3]) {
+  const V f = sp(f61);
+  const int64_t q = mad(f.h, f.h, mad(f.h + f.h, f.l, mad(f.l, f.l, 0) >> 32) >> 32);  // f^2
+  const int64_t t = q + (1ll << 56), u = f61 >> 3;
+  w[0] = sp((int64_t)((uint64_t)((t - u) & ~1ll) << (k - 1)));
+  w[1] = sp((int64_t)((uint64_t)((3ll << 56) - q) << k));
+  w[2] = sp((int64_t)((uint64_t)((t + u) & ~1ll) << (k - 1)));
+}
+
 // base + k v for a small integer k.
 FX_HD int64_t kmad(int k, V v, int64_t base) {
   const int64_t r = mad(v.l, k, base);

@@ -501,7 +501,7 @@ template <int KF, bool EXT, bool KSMEM>
 static int launch_pass(orbit_bunch_t* bu, cudaStream_t s, size_t smem, const DevOp* ops, int a, int b,
                        const MapCtx& m, const KickArgs& ka, ScState* ext, const SetupArgs& sa, double* knl_buf,
                        int km, bool fixed, const PassPrep* prep) {
-  int threads = fixed ? ORBIT_FX_THREADS : ORBIT_PASS_THREADS;
+  const int threads = spread_threads(bu->n, fixed ? ORBIT_FX_THREADS : ORBIT_PASS_THREADS);
   int bps = KSMEM ? (int)(kPassSmem / (smem > 0 ? smem : 1)) : 4;
   if (bps < 1) bps = 1;
   if (bps > 4) bps = 4;

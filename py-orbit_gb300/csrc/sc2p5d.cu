@@ -20,7 +20,10 @@ static const int kMaxSmem = 220 * 1024;
 // Thread bound of the single-bunch shared-memory deposit (one block per SM
 // holds the 128x128 grid): 65536 / ORBIT_DEP_THREADS registers per thread.
 #ifndef ORBIT_DEP_THREADS
-#define ORBIT_DEP_THREADS 768
+#define ORBIT_DEP_THREADS 1024
+#endif
+#ifndef ORBIT_MIN_THREADS
+#define ORBIT_MIN_THREADS 256
 #endif
 
 bool make_fft_plan(int n, FftPlan& pl) {
@@ -686,27 +689,29 @@ __global__ void k_rb_analysis(ScState* st, const double* __restrict__ rho, const
   }
 }
 
+// Clears n words of the block's dynamic shared memory (16-byte aligned).
+__device__ __forceinline__ void zero_shared(unsigned* p, int n) {
+  for (int i = threadIdx.x; i < n >> 2; i += blockDim.x) reinterpret_cast<uint4*>(p)[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = (n & ~3) + threadIdx.x; i < n; i += blockDim.x) p[i] = 0u;
+}
+
 // Deposit, plain form.  SMEM: block-private fixed-point grids in shared
 // memory, flushed with one 64-bit atomic per non-zero cell.  With K > 0
 // (uniform macrosize) each particle deposits unit weight in units of 2^-K
 // through the integer path (deposit_fixed); otherwise, and for the rare
 // particle the integer path declines, macrosize * qscale through FP64.
-// Blocks of up to 768 threads (80 registers: 24 warps per SM) cover the
-// latency of the shared-memory atomics; 1024 threads at 64 registers spill
-// and ran slower.
+// Blocks of up to 1024 threads (64 registers) cover the latency of the
+// shared-memory atomics: 333,333 particles 133 us a whole kick against 138 with
+// 768.
 template <bool SMEM>
 __device__ __forceinline__ void deposit_plain_body(const double* __restrict__ x, const double* __restrict__ y,
                                                    const double* __restrict__ z, const double* __restrict__ msize,
                                                    int n, const ScState* st, unsigned long long* g_rho,
                                                    unsigned long long* g_z, double ms_uniform, double qscale, int nx,
                                                    int ny, int nz, int K, int blk, int nblk) {
-  DepConst d;
-  load_dep_const(d, st, nx, ny, nz);
-  if (d.skip) return;
-  DepFix df;
-  if (K > 0) load_dep_fix(df, st, nx, ny, nz, K);
+  if (st->skip) return;
   // shared: low words of the nx*ny + nz cells, then their high words
-  extern __shared__ unsigned s_acc32[];
+  extern __shared__ __align__(16) unsigned s_acc32[];
   const int ncell = nx * ny + nz;
   GridAcc<SMEM> rho, zg;
   if constexpr (SMEM) {
@@ -714,18 +719,19 @@ __device__ __forceinline__ void deposit_plain_body(const double* __restrict__ x,
     rho.hi_off = ncell;
     zg.lo = s_acc32 + nx * ny;
     zg.hi_off = ncell;
-    for (int i = threadIdx.x; i < 2 * ncell; i += blockDim.x) s_acc32[i] = 0u;
-    __syncthreads();
   } else {
     rho.p = g_rho;
     zg.p = g_z;
   }
-  for (int i = blk * blockDim.x + threadIdx.x; i < n; i += nblk * blockDim.x) {
-    double xi = x[i], yi = y[i], zi = z[i];
-    if (K > 0 && deposit_fixed(df, rho, zg, xi, yi, zi)) continue;
-    double ms = msize ? msize[i] * qscale : ms_uniform;
-    deposit_plain(d, rho, zg, xi, yi, zi, ms);
+  __shared__ DepFast s_d;
+  __shared__ DepSlow<GridAcc<SMEM>, GridAcc<SMEM>> s_s;
+  if (threadIdx.x < 3) load_dep_fast(&s_d, st, nx, ny, nz, K, n);
+  if (threadIdx.x == 32) {
+    s_s = {rho, zg, st, {x, y, z}, msize, ms_uniform, qscale, nx, ny, nz, K};
   }
+  if constexpr (SMEM) zero_shared(s_acc32, 2 * ncell);
+  __syncthreads();
+  deposit_particles(&s_d, &s_s, rho, zg, x, y, z, msize, n, qscale, nx, ny, nz, K, blk, nblk);
   if constexpr (SMEM) {
     __syncthreads();
     for (int i = threadIdx.x; i < ncell; i += blockDim.x) {
@@ -756,16 +762,12 @@ __device__ __forceinline__ void deposit_band_body(const double* __restrict__ x, 
                                                   int n, const ScState* st, unsigned long long* g_rho,
                                                   unsigned long long* g_z, double ms_uniform, double qscale, int nx,
                                                   int ny, int nz, int K, int rpb, int band, int chunk, int nchunk) {
-  DepConst d;
-  load_dep_const(d, st, nx, ny, nz);
-  if (d.skip) return;
-  DepFix df;
-  if (K > 0) load_dep_fix(df, st, nx, ny, nz, K);
+  if (st->skip) return;
   const int r0 = band * rpb, r1 = min(nx, r0 + rpb);
   const int lr0 = max(r0 - 1, 0), lr1 = min(r1 + 1, nx);
   const int nloc = (lr1 - lr0) * ny;
   const int ncell = nloc + nz;
-  extern __shared__ unsigned s_band32[];
+  extern __shared__ __align__(16) unsigned s_band32[];
   BandAcc rho;
   rho.lo = s_band32;
   rho.hi_off = ncell;
@@ -776,14 +778,18 @@ __device__ __forceinline__ void deposit_band_body(const double* __restrict__ x, 
   GridAcc<true> zg;
   zg.lo = s_band32 + nloc;
   zg.hi_off = ncell;
-  for (int i = threadIdx.x; i < 2 * ncell; i += blockDim.x) s_band32[i] = 0u;
-  __syncthreads();
-  for (int i = chunk * blockDim.x + threadIdx.x; i < n; i += nchunk * blockDim.x) {
-    double xi = x[i], yi = y[i], zi = z[i];
-    if (K > 0 && deposit_fixed(df, rho, zg, xi, yi, zi)) continue;
-    double ms = msize ? msize[i] * qscale : ms_uniform;
-    deposit_plain(d, rho, zg, xi, yi, zi, ms);
+  __shared__ DepFast s_d;
+  __shared__ DepSlow<BandAcc, GridAcc<true>> s_s;
+  if (threadIdx.x < 3) load_dep_fast(&s_d, st, nx, ny, nz, K, n);
+  if (threadIdx.x == 32) {
+    s_s = {rho, zg, st, {x, y, z}, msize, ms_uniform, qscale, nx, ny, nz, K};
   }
+  __shared__ BandKeys s_k;
+  __shared__ int s_queue[64 * (768 / 32)];
+  if (threadIdx.x == 64) load_band_keys(&s_k, st, nx, rho);
+  zero_shared(s_band32, 2 * ncell);
+  __syncthreads();
+  deposit_band_particles(&s_d, &s_s, &s_k, s_queue, rho, zg, x, y, z, msize, n, qscale, nx, ny, nz, K, chunk, nchunk);
   __syncthreads();
   for (int i = threadIdx.x; i < ncell; i += blockDim.x) {
     unsigned long long v = ((unsigned long long)s_band32[ncell + i] << 32) | s_band32[i];
@@ -1138,13 +1144,26 @@ static int ext_blocks(int n) {
   return b < 1 ? 1 : (b > cap ? cap : b);
 }
 
+// Threads a block of a particle kernel of at most `most`: a bunch too small to
+// fill every SM with such blocks spreads over more of them in smaller blocks.
+// 16 kicks of 20,011 particles on 64 x 64 x 32: 866 us with at least 256
+// threads, 893 with 128 (more copies of the grid) and with 512 (half the SMs
+// idle).  The separate kick kernel keeps its size: 1e4 particles, one kick, 63.6
+// against 68.0 us.
+int spread_threads(int n, int most) {
+  int t = ((n + num_sms() - 1) / num_sms() + 31) & ~31;
+  t = t < ORBIT_MIN_THREADS ? ORBIT_MIN_THREADS : t;
+  return t < most ? t : most;
+}
+
 // launch geometry for particle kernels that keep a grid copy in shared memory
-static void particle_geometry(size_t smem, int n, int max_threads, int* blocks, int* threads) {
+static void particle_geometry(size_t smem, int n, int max_threads, bool spread, int* blocks, int* threads) {
   int bps = smem > 0 ? (int)(kMaxSmem / smem) : 8;
   if (bps < 1) bps = 1;
   if (bps > 4) bps = 4;
   *threads = (bps == 1) ? 1024 : 512;
   if (*threads > max_threads) *threads = max_threads & ~31;  // register-limited kernels
+  if (spread) *threads = spread_threads(n, *threads);
   int b = num_sms() * bps;
   int need = (n + *threads - 1) / *threads;
   *blocks = need < b ? (need < 1 ? 1 : need) : b;
@@ -1650,7 +1669,7 @@ int sc_enqueue_kick(orbit_sc2p5d_t* c, orbit_bunch_t* b, double length, cudaStre
   size_t sm = sizeof(unsigned long long) * ((size_t)c->nx * c->ny + c->nz);
   int blocks, threads;
   const int* mt_dep = particle_kernel_threads();
-  particle_geometry(c->smem_deposit ? sm : 0, n, mt_dep[c->smem_deposit ? 0 : 1], &blocks, &threads);
+  particle_geometry(c->smem_deposit ? sm : 0, n, mt_dep[c->smem_deposit ? 0 : 1], true, &blocks, &threads);
   ORBIT_PB("deposit", s);
   {
     if (c->smem_deposit) {
@@ -1776,8 +1795,8 @@ int sc_enqueue_kick(orbit_sc2p5d_t* c, orbit_bunch_t* b, double length, cudaStre
     BndShape bshape = bnd_shape_of(bnd);
     size_t smk = (plain ? sizeof(double) : sizeof(float)) * ((size_t)c->nx * c->ny + c->nz);
     const int* mt_kick = particle_kernel_threads() + 2;
-    particle_geometry(c->smem_kick ? smk : 0, n, mt_kick[(plain ? 0 : 2) + (c->smem_kick ? 0 : 1)], &blocks,
-                      &threads);
+    particle_geometry(c->smem_kick ? smk : 0, n, mt_kick[(plain ? 0 : 2) + (c->smem_kick ? 0 : 1)], false,
+                      &blocks, &threads);
     ORBIT_PB("kick", s);
     if (plain) {
       if (c->smem_kick)

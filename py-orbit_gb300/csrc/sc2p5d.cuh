@@ -217,6 +217,7 @@ int sc_enqueue_kick(orbit_sc2p5d_t* c, orbit_bunch_t* b, double length, cudaStre
 cudaError_t sc_order_before(orbit_sc2p5d_t* c, cudaStream_t s);
 cudaError_t sc_mark_used(orbit_sc2p5d_t* c, cudaStream_t s);
 DepScales sc_dep_scales(const orbit_sc2p5d_t* c, const orbit_bunch_t* b);
+int spread_threads(int n, int most);
 SetupArgs sc_setup_args(const orbit_sc2p5d_t* c, const DepScales& d, const orbit_boundary* bnd = nullptr);
 // The boundary's inside test (type -1 for none).
 BndShape bnd_shape_of(const orbit_boundary* bnd);

@@ -544,10 +544,35 @@ __device__ __forceinline__ void load_dep_const(DepConst& d, const ScState* st, i
 // the low word wraps modulo 2^32 and the add that wraps carries 1 into the
 // high word, so hi * 2^32 + lo, read once all adds are done, is the exact
 // sum modulo 2^64.
+//
+// row(i) addresses cell i for adds at i + j with j known to the compiler.
 template <bool SHARED> struct GridAcc;
+
+// v at the low word lo and the high word hi of a cell, as shared-memory
+// addresses: two atomics and the carry between them (left to atomicAdd and a
+// test for a high word of zero, a cell takes a branch besides).
+__device__ __forceinline__ void add_lo_hi(unsigned lo, unsigned hi, unsigned long long v) {
+  asm volatile(
+      "{\n\t.reg .u32 o, c, h;\n\t"
+      "atom.shared.add.u32 o, [%0], %2;\n\t"
+      "add.cc.u32 c, o, %2;\n\t"
+      "addc.u32 h, %3, 0;\n\t"
+      "red.shared.add.u32 [%1], h;\n\t}" ::"r"(lo),
+      "r"(hi), "r"((unsigned)v), "r"((unsigned)(v >> 32))
+      : "memory");
+}
+struct SharedRow {
+  unsigned lo, hi;
+  __device__ __forceinline__ void add(int j, unsigned long long v) const { add_lo_hi(lo + 4 * j, hi + 4 * j, v); }
+};
 
 template <> struct GridAcc<false> {
   unsigned long long* p;
+  struct Row {
+    unsigned long long* p;
+    __device__ __forceinline__ void add(int j, unsigned long long v) const { atomicAdd(p + j, v); }
+  };
+  __device__ __forceinline__ Row row(int i) const { return Row{p + i}; }
   __device__ __forceinline__ void add(int i, unsigned long long v) const { atomicAdd(p + i, v); }
   // every particle is deposited by the block that reads it
   __device__ __forceinline__ bool owns(int) const { return true; }
@@ -557,12 +582,11 @@ template <> struct GridAcc<false> {
 template <> struct GridAcc<true> {
   unsigned* lo;  // low words; the high words are at lo + hi_off
   int hi_off;
-  __device__ __forceinline__ void add(int i, unsigned long long v) const {
-    unsigned l = (unsigned)v, h = (unsigned)(v >> 32);
-    unsigned old = atomicAdd(lo + i, l);
-    h += (old + l < old) ? 1u : 0u;
-    if (h) atomicAdd(lo + hi_off + i, h);
+  __device__ __forceinline__ SharedRow row(int i) const {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(lo) + 4 * i;
+    return SharedRow{a, a + 4 * hi_off};
   }
+  __device__ __forceinline__ void add(int i, unsigned long long v) const { row(i).add(0, v); }
   __device__ __forceinline__ unsigned long long get(int i) const {
     return ((unsigned long long)lo[hi_off + i] << 32) | lo[i];
   }
@@ -582,13 +606,11 @@ struct BandAcc {
   int base;
   int r0, r1;
   bool first;
-  __device__ __forceinline__ void add(int i, unsigned long long v) const {
-    i -= base;
-    unsigned l = (unsigned)v, h = (unsigned)(v >> 32);
-    unsigned old = atomicAdd(lo + i, l);
-    h += (old + l < old) ? 1u : 0u;
-    if (h) atomicAdd(lo + hi_off + i, h);
+  __device__ __forceinline__ SharedRow row(int i) const {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(lo) + 4 * (i - base);
+    return SharedRow{a, a + 4 * hi_off};
   }
+  __device__ __forceinline__ void add(int i, unsigned long long v) const { row(i).add(0, v); }
   __device__ __forceinline__ unsigned long long get(int i) const {
     return ((unsigned long long)lo[hi_off + i] << 32) | lo[i];
   }
@@ -786,6 +808,266 @@ __device__ __forceinline__ bool deposit_fixed(const DepFix& d, const RA& rho, co
     }
   }
   return true;
+}
+
+// The constants of a block's deposit: v 2^F is the coordinate in cells plus
+// 1/2, x a + c for a uniform macrosize and (x - c) a + 2^(F-1) for others (as
+// deposit_fixed and deposit_plain round it), its high word within [lo, lo + span] where the particle is
+// surely inside the grid's limits.
+struct DepFast {
+  double a[3], c[3];
+  int F[3], lo[3];
+  unsigned span[3];
+  int none;               // every particle goes the general way
+  double min[3], max[3];  // the limits themselves
+};
+
+// g: extra bits of a per-particle macrosize (K = 0): about 2^58 units at the
+// mean of n particles; 0: none fit, every particle goes the general way.
+__host__ __device__ __forceinline__ int dep_ms_bits(int n) {
+  int b = 0;
+  while (b < 30 && (n >> (b + 1)) != 0) ++b;
+  return b >= 9 ? b - 4 : 0;
+}
+
+// Executed by lanes 0..2 of one warp, one coordinate each.
+__device__ __forceinline__ void load_dep_fast(DepFast* d, const ScState* st, int nx, int ny, int nz, int K, int n) {
+  const int k = threadIdx.x;
+  const int nc = k == 0 ? nx : k == 1 ? ny : nz;
+  const double inv = k == 0 ? st->inv_dx : k == 1 ? st->inv_dy : st->inv_dz;
+  const double mn = k == 0 ? st->xmin : k == 1 ? st->ymin : st->zmin;
+  const int F = fix_bits(nc);
+  const double scale = __hiloint2double((1023 + F) << 20, 0);
+  const double c = 0.5 - mn * inv;
+  d->a[k] = inv * scale;
+  d->c[k] = K > 0 ? c * scale : mn;
+  d->F[k] = F;
+  d->min[k] = mn;
+  d->max[k] = k == 0 ? st->xmax : k == 1 ? st->ymax : st->zmax;
+  // cells [0, n - 1] of x and y, [0, nz] of z, less 2^(32 - F) at each end: far
+  // above the rounding of v unless the grid lies 2^16 cells off the origin
+  const int lo = (1 << (F - 33)) + 1;
+  const int hi = (int)((((long long)nc << F) - (1ll << (F - 1))) >> 32) + (k == 2 ? 1 << (F - 32) : 0) - 1;
+  d->lo[k] = lo;
+  d->span[k] = (unsigned)(hi - lo);
+  const bool ok = (K > 0 ? fabs(c) < 65536.0 : dep_ms_bits(n) > 0) && hi >= lo;
+  const bool all = __all_sync(7u, ok);
+  if (k == 0) d->none = !all;
+}
+
+// A particle next to a limit: inside all three, and its cell coordinate where
+// deposit_fixed takes it.
+static __device__ __noinline__ bool dep_edge(const DepFast* d, double x, double y, double z, int hx, int hy, int hz) {
+  const double v[3] = {x, y, z};
+  const int h[3] = {hx, hy, hz};
+  bool in = true;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int q = 1 << (d->F[k] - 34);  // a quarter cell
+    in = in && v[k] >= d->min[k] && v[k] <= d->max[k] && h[k] >= q && h[k] < d->lo[k] + (int)d->span[k] + q;
+  }
+  return in;
+}
+
+// One particle inside the grid.  MS: M is its macrosize in units of
+// 2^-(g) / S, else every particle counts 2^K.  The sums are deposit_fixed's,
+// bit for bit, for K > 0.  Returns false, with nothing done, for the others.
+//
+// Bound by the issue of instructions (with the fields of the doubles taken
+// apart, keys compared and every product formed from unsigned halves a particle
+// took 740): the conversions run on the otherwise idle FP64 pipe (three
+// multiply-adds and three conversions, 64 clocks a warp each), one square gives
+// the three weights, and the nine products take four multiply-adds each.  1e6
+// particles, 128 x 128 x 64: 44 -> 27 us; 333,333 with their own macrosizes on
+// 96 x 80 x 48, whose FP64 sums became integer ones: 60 -> 25 us.
+template <bool MS, class RA, class ZA>
+__device__ __forceinline__ bool deposit_fast(const DepFast& d, const DepFast* sd, const RA& rho, const ZA& zg, double x, double y,
+                                             double z, long long M, int nx, int ny, int nz, int K) {
+  auto cells = [&](double v, int k) -> long long {
+    if (MS) return __double2ll_rz((v - d.c[k]) * d.a[k]) + (1ll << (d.F[k] - 1));
+    return __double2ll_rz(fma(v, d.a[k], d.c[k]));
+  };
+  const long long vx = cells(x, 0), vy = cells(y, 1), vz = cells(z, 2);
+  const int hx = (int)(vx >> 32), hy = (int)(vy >> 32), hz = (int)(vz >> 32);
+  const bool in = ((unsigned)(hx - d.lo[0]) <= d.span[0]) & ((unsigned)(hy - d.lo[1]) <= d.span[1]) &
+                  ((unsigned)(hz - d.lo[2]) <= d.span[2]);
+  if (!in && !dep_edge(sd, x, y, z, hx, hy, hz)) return false;
+  if (MS && !fx::within(M, 1 << 29)) return false;
+  const int ix = min(max(hx >> (d.F[0] - 32), 1), nx - 2), iy = min(max(hy >> (d.F[1] - 32), 1), ny - 2);
+  if (!rho.owns(ix)) return true;  // another block's particle
+  // f = v - i - 1/2 in Q61, to 2^-56
+  auto frac = [](long long v, int F, int i) {
+    const unsigned long long t = (unsigned long long)v << (62 - F);
+    const long long f = (long long)(t - ((unsigned long long)(unsigned)((i << 30) + (1 << 29)) << 32));
+    return (f >> 1) & ~31ll;
+  };
+  fx::V wx[3], wy[3];
+  fx::tsc_weights_q58(frac(vx, d.F[0], ix), 4, wx);
+  fx::tsc_weights_q58(frac(vy, d.F[1], iy), 1, wy);
+  const fx::V m = fx::sp(M);
+  int sh = 57 - K;  // products Wx Wy in Q57
+  if (MS) {
+    sh = K - 4;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) wx[i] = fx::sp(fx::mul_floor(wx[i], m) << 3);  // 2 Wx M
+  }
+  const int half = 1 << (sh - 1);  // sh <= 28
+  const int base = (ix - 1) * ny + (iy - 1);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const auto row = rho.row(base + i * ny);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) row.add(j, (unsigned long long)(fx::mul_floor_r(wx[i], wy[j], half) >> sh));
+  }
+  if (nz > 1) {
+    const int iz = hz >> (d.F[2] - 32);
+    const long long w = (long long)(((unsigned long long)vz << (62 - d.F[2])) -
+                                    ((unsigned long long)(unsigned)(iz << 30) << 32));  // Q62
+    const int i0 = iz == 0 ? nz - 1 : iz - 1, ip = iz >= nz ? 0 : iz;
+    if (MS) {
+      const long long hz2 = 1ll << (K - 3);
+      zg.add(i0, (unsigned long long)(fx::mul_floor(fx::sp((1ll << 62) - w), m, hz2) >> (K - 2)));
+      zg.add(ip, (unsigned long long)(fx::mul_floor(fx::sp(w), m, hz2) >> (K - 2)));
+    } else {
+      const int sz = 56 - K;
+      const long long hz1 = 1ll << (sz - 1), wp = w >> 6;
+      zg.add(i0, (unsigned long long)(((1ll << 56) - wp + hz1) >> sz));
+      zg.add(ip, (unsigned long long)((wp + hz1) >> sz));
+    }
+  } else {
+    zg.add(0, MS ? (unsigned long long)((M + (1ll << (K - 1))) >> K) : 1ull << K);
+  }
+  return true;
+}
+
+// A particle outside the grid, or whose macrosize is far above the mean: the
+// general way.
+template <class RA, class ZA>
+struct DepSlow {
+  RA rho;
+  ZA zg;
+  const ScState* st;
+  const double* c[3];
+  const double* msize;
+  double ms_uniform, qscale;
+  int nx, ny, nz, K;
+};
+
+template <class RA, class ZA>
+__device__ __noinline__ void deposit_slow(const DepSlow<RA, ZA>* s, int i) {
+  const double x = s->c[0][i], y = s->c[1][i], z = s->c[2][i];
+  if (s->K > 0) {
+    DepFix df;
+    load_dep_fix(df, s->st, s->nx, s->ny, s->nz, s->K);
+    if (deposit_fixed(df, s->rho, s->zg, x, y, z)) return;
+  }
+  DepConst d;
+  load_dep_const(d, s->st, s->nx, s->ny, s->nz);
+  deposit_plain(d, s->rho, s->zg, x, y, z, s->msize ? s->msize[i] * s->qscale : s->ms_uniform);
+}
+
+// Deposits particle i one way or the other.  g: dep_ms_bits, q: qscale 2^g.
+template <class RA, class ZA>
+__device__ __forceinline__ void deposit_one(const DepFast& d, const DepFast* sd, const DepSlow<RA, ZA>* ss,
+                                            const RA& rho, const ZA& zg, const double* __restrict__ x,
+                                            const double* __restrict__ y, const double* __restrict__ z,
+                                            const double* __restrict__ msize, int g, double q, int nx, int ny, int nz,
+                                            int K, int i) {
+  const bool done = K > 0 ? deposit_fast<false>(d, sd, rho, zg, x[i], y[i], z[i], 0, nx, ny, nz, K)
+                          : deposit_fast<true>(d, sd, rho, zg, x[i], y[i], z[i], __double2ll_rn(msize[i] * q), nx, ny,
+                                               nz, g);
+  if (!done) deposit_slow(ss, i);
+}
+
+// The particles blk * blockDim + thread, ... of a block's deposit.
+template <class RA, class ZA>
+__device__ __forceinline__ void deposit_particles(const DepFast* sd, const DepSlow<RA, ZA>* ss, const RA& rho,
+                                                  const ZA& zg, const double* __restrict__ x,
+                                                  const double* __restrict__ y, const double* __restrict__ z,
+                                                  const double* __restrict__ msize, int n, double qscale, int nx,
+                                                  int ny, int nz, int K, int blk, int nblk) {
+  const DepFast d = *sd;
+  const int i0 = blk * blockDim.x + threadIdx.x, di = nblk * blockDim.x, g = dep_ms_bits(n);
+  const double q = sf::pow2mul(qscale, g);
+  if (d.none) {
+    for (int i = i0; i < n; i += di) deposit_slow(ss, i);
+  } else if (K > 0) {  // two loops: the test stays outside
+    for (int i = i0; i < n; i += di) deposit_one(d, sd, ss, rho, zg, x, y, z, msize, g, q, nx, ny, nz, K, i);
+  } else {
+    for (int i = i0; i < n; i += di) deposit_one(d, sd, ss, rho, zg, x, y, z, msize, g, q, nx, ny, nz, 0, i);
+  }
+}
+
+// Which particles a band looks at, by the order of the high words of the
+// doubles alone (widened by 1/16 cell, so none of its own is missed): those
+// whose centre row may be its own, and for the first band also those that may
+// lie outside the transverse grid.
+struct BandKeys {
+  int xlo, xhi, ylo, yhi, xout;
+};
+
+__device__ __forceinline__ int hi_key(double v) {
+  const int h = __double2hiint(v);
+  return h ^ ((h >> 31) & 0x7fffffff);
+}
+
+__device__ __forceinline__ void load_band_keys(BandKeys* k, const ScState* st, int nx, const BandAcc& a) {
+  const double dx = 1.0 / st->inv_dx, dy = 1.0 / st->inv_dy;
+  k->xlo = a.first ? -0x7fffffff - 1 : hi_key(st->xmin + (a.r0 - 0.5625) * dx);
+  k->xhi = a.r1 >= nx ? 0x7fffffff : hi_key(st->xmin + (a.r1 - 0.4375) * dx);
+  k->ylo = a.first ? hi_key(st->ymin + 0.0625 * dy) : -0x7fffffff - 1;
+  k->yhi = a.first ? hi_key(st->ymax - 0.0625 * dy) : 0x7fffffff;
+  k->xout = a.first ? hi_key(st->xmax - 0.0625 * dx) : 0x7fffffff;
+}
+
+// The same particles for a band: a warp sets aside those that may be the
+// band's own until it has 32, and deposits them together.  With every lane
+// testing and depositing its own, a warp went through the whole deposit in
+// every band for the lanes that own theirs: 835 against 572 us for 16e6
+// particles on 256 x 256 in three bands.
+static __device__ __forceinline__ void deposit_band_particles(const DepFast* sd, const DepSlow<BandAcc, GridAcc<true>>* ss,
+                                                       const BandKeys* bk, int* queue, const BandAcc& rho,
+                                                       const GridAcc<true>& zg, const double* __restrict__ x,
+                                                       const double* __restrict__ y, const double* __restrict__ z,
+                                                       const double* __restrict__ msize, int n, double qscale, int nx,
+                                                       int ny, int nz, int K, int blk, int nblk) {
+  const DepFast d = *sd;
+  const BandKeys k = *bk;
+  const int lane = threadIdx.x & 31, g = dep_ms_bits(n);
+  const double q = sf::pow2mul(qscale, g);
+  int* mine = queue + 64 * (threadIdx.x >> 5);
+  int have = 0;
+  auto flush = [&](int cnt) {
+    __syncwarp();
+    if (lane < cnt) {
+      const int i = mine[lane];
+      if (d.none) deposit_slow(ss, i);
+      else if (K > 0) deposit_one(d, sd, ss, rho, zg, x, y, z, msize, g, q, nx, ny, nz, K, i);
+      else deposit_one(d, sd, ss, rho, zg, x, y, z, msize, g, q, nx, ny, nz, 0, i);
+    }
+    __syncwarp();
+  };
+  const int di = nblk * blockDim.x;
+  for (int i = blk * blockDim.x + threadIdx.x; i - lane < n; i += di) {
+    bool own = false;
+    if (i < n) {
+      const int kx = hi_key(x[i]);
+      own = kx >= k.xlo && kx <= k.xhi;
+      if (rho.first && !own) {
+        const int ky = hi_key(y[i]);
+        own = kx >= k.xout || ky <= k.ylo || ky >= k.yhi;
+      }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, own);
+    if (own) mine[have + __popc(m & ((1u << lane) - 1u))] = i;
+    have += __popc(m);
+    if (have >= 32) {
+      flush(32);
+      have -= 32;
+      if (lane < have) mine[lane] = mine[32 + lane];
+    }
+  }
+  flush(have);
 }
 
 // Fixed-point kick: phi and lambda as 64-bit integers with per-kick scales
