@@ -470,6 +470,204 @@ __global__ void __launch_bounds__(128) k_conv3_tcb(const float* __restrict__ in,
   }
 }
 
+// Weight and bias gradients of a 3x3 layer on the tensor cores, for images
+// whose pixels come in whole groups of 32 (H W % 32 = 0, W % 4 = 0) and layers
+// of CI | cin inputs: CTA (chunk, slice) takes CI input channels of one kernel
+// row ky, so that the three taps of the row read the same pixels.  The product
+// is M = 128 (rows o < COUT, the rest zero) x N = 3 CI (column 32-pixel dot
+// products of tap kx and channel ci at kx * CI + ci), its K a slice of 32-pixel
+// stages, accumulated in TMEM; the next stage's loads overlap the MMAs.
+//
+// Eight rows (channels) x 32 pixels of an operand are one warp's work: lane
+// (row r = lane % 8, group g = lane / 8) loads 8 consecutive pixels as two
+// float4, takes the pixels to the left and right of its own from the
+// neighbouring groups' registers (the outer groups load them), and writes the
+// three taps' rows as float4 without bank conflicts.  With one thread a row of
+// 16 or 32 scalar loads (k_conv3_wgrad_tc) every load instruction touched 32
+// lines and the L1 bounded it: 48 -> 16 channels on 16 images of 128 x 128
+// 426 us; a training step 3820 us, this 2723 (2853 and 2938 with six and eight
+// CTAs per SM in the grid instead of four).
+template <int CI, int COUT>
+__global__ void __launch_bounds__(128) k_conv3_wgrad_row(const float* __restrict__ x, int cin,
+                                                         const float* __restrict__ dy, int H, int W, int nb, int spc,
+                                                         float* __restrict__ dw, float* __restrict__ db, int* err,
+                                                         TcWait tw) {
+  constexpr int N = 3 * CI, NB = CI / 8, NA = COUT / 8, NG = (NA + NB + 3) / 4;  // groups of 8 rows, per warp
+  constexpr uint32_t COLS = N <= 64 ? 64u : 128u;
+  extern __shared__ unsigned char tc_raw[];
+  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane & 7, g = lane >> 3;
+  const uint32_t raw = smem_u32(tc_raw);
+  const uint32_t sA = (raw + 1023u) & ~1023u, sB = sA + kTcStageA;
+  unsigned char* gA = tc_raw + (sA - raw);
+  const int HW = H * W, K9 = 9 * cin;
+  const int ky = (int)blockIdx.x % 3, c0 = ((int)blockIdx.x / 3) * CI;
+  const int total = nb * (HW / kTcKC);           // stages of the batch
+  const int st0 = blockIdx.y * spc, nst = min(spc, total - st0);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                 "r"(COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar)));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  // rows COUT.. of A stay zero
+  for (int i = tid + COUT / 8 * 64; i < 128 / 8 * 64; i += 128)
+    reinterpret_cast<float4*>(gA)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = s_tmem;
+  float v[NG][8], eL[NG], eR[NG];
+  unsigned mL = 0u, mR = 0u, mC = 0u;  // bit e: pixel e's left, right, centre neighbour is in the image
+  float bsum[NG];
+#pragma unroll
+  for (int k = 0; k < NG; ++k) bsum[k] = 0.f;
+  auto load_stage = [&](int st) {
+    const int img = st / (HW / kTcKC), q0 = (st - img * (HW / kTcKC)) * kTcKC + 8 * g;
+    int py = q0 / W, px = q0 - py * W;
+    mL = mR = mC = 0u;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const unsigned in = (unsigned)(py + ky - 1) < (unsigned)H ? 1u : 0u;
+      mC |= in << e;
+      mL |= (px > 0 ? in : 0u) << e;
+      mR |= (px + 1 < W ? in : 0u) << e;
+      if (++px == W) {
+        px = 0;
+        ++py;
+      }
+    }
+    const int sh = (ky - 1) * W;
+#pragma unroll
+    for (int k = 0; k < NG; ++k) {
+      const int grp = warp + 4 * k;
+      eL[k] = eR[k] = 0.f;
+      if (grp < NA) {  // dy rows
+        const float4* src = reinterpret_cast<const float4*>(dy + ((size_t)img * COUT + grp * 8 + r) * HW + q0);
+        const float4 a = __ldg(src), b = __ldg(src + 1);
+        v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
+        v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
+      } else if (grp < NA + NB) {  // x rows, shifted by the kernel row
+        const float* base = x + ((size_t)img * cin + c0 + (grp - NA) * 8 + r) * HW;
+        const int q = q0 + sh;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        // four pixels of a row at a time: all in the image or none (W % 4 = 0)
+        if (mC & 1u) a = __ldg(reinterpret_cast<const float4*>(base + q));
+        if (mC & 16u) b = __ldg(reinterpret_cast<const float4*>(base + q + 4));
+        v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
+        v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
+        if (g == 0 && (mL & 1u)) eL[k] = __ldg(base + q - 1);
+        if (g == 3 && (mR & 128u)) eR[k] = __ldg(base + q + 8);
+      }
+    }
+  };
+  bool ok = true;
+  int s = 0;
+  load_stage(st0);
+  for (; s < nst; ++s) {
+#pragma unroll
+    for (int k = 0; k < NG; ++k) {
+      const int grp = warp + 4 * k;
+      if (grp < NA) {
+        unsigned char* row = gA + grp * 1024 + r * 16 + g * 256;
+        if (blockIdx.x == 0) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) bsum[k] += v[k][e];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          *reinterpret_cast<float4*>(row + u * 128) = make_float4(to_tf32(v[k][4 * u]), to_tf32(v[k][4 * u + 1]),
+                                                                  to_tf32(v[k][4 * u + 2]), to_tf32(v[k][4 * u + 3]));
+      } else if (grp < NA + NB) {
+        float t[10];  // the pixels q0 - 1 .. q0 + 8
+        const float lf = __shfl_up_sync(0xffffffffu, v[k][7], 8), rt = __shfl_down_sync(0xffffffffu, v[k][0], 8);
+        t[0] = to_tf32(g == 0 ? eL[k] : lf);
+        t[9] = to_tf32(g == 3 ? eR[k] : rt);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) t[e + 1] = to_tf32(v[k][e]);
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx) {
+          const unsigned m = kx == 0 ? mL : kx == 1 ? mC : mR;
+          unsigned char* row = gA + kTcStageA + (kx * NB + grp - NA) * 1024 + r * 16 + g * 256;
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            *reinterpret_cast<float4*>(row + u * 128) =
+                make_float4(m >> (4 * u) & 1u ? t[4 * u + kx] : 0.f, m >> (4 * u + 1) & 1u ? t[4 * u + kx + 1] : 0.f,
+                            m >> (4 * u + 2) & 1u ? t[4 * u + kx + 2] : 0.f,
+                            m >> (4 * u + 3) & 1u ? t[4 * u + kx + 3] : 0.f);
+        }
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (tid == 0 && !tw.withhold) {
+#pragma unroll
+      for (int j = 0; j < kTcKC / 8; ++j) {
+        const uint64_t ad = tc_desc(sA + 256u * j), bd = tc_desc(sB + 256u * j);
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+            "l"(ad), "l"(bd), "r"(tc_idesc(N)), "r"((s > 0 || j > 0) ? 1u : 0u));
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                       smem_u32(&s_bar))
+                   : "memory");
+    }
+    if (s + 1 < nst) load_stage(st0 + s + 1);
+    ok = __syncthreads_and(mbar_wait_bounded(smem_u32(&s_bar), (uint32_t)(s & 1), tw.cycles));
+    if (!ok) break;
+  }
+  if (!ok) {
+    if (tid == 0) atomicOr(err, 1);
+    if (!tw.withhold &&
+        !__syncthreads_and(mbar_wait_bounded(smem_u32(&s_bar), (uint32_t)(s & 1), tw.cycles)) && tid == 0)
+      atomicOr(err, 2);
+  }
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (ok) {
+    // row o = tid of D: TMEM lane 32 * warp + lane
+#pragma unroll
+    for (int n0 = 0; n0 < N; n0 += 16) {
+      uint32_t q[16];
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]),
+            "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
+          : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)n0));
+      asm volatile("tcgen05.wait::ld.sync.aligned;");
+      if (tid < COUT) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int kx = (n0 + j) / CI, ci = c0 + (n0 + j) % CI;
+          atomicAdd(dw + (size_t)tid * K9 + ci * 9 + ky * 3 + kx, __uint_as_float(q[j]));
+        }
+      }
+    }
+    if (blockIdx.x == 0) {
+#pragma unroll
+      for (int k = 0; k < NG; ++k) {
+        const int grp = warp + 4 * k;
+        float b = bsum[k];
+        b += __shfl_xor_sync(0xffffffffu, b, 8);
+        b += __shfl_xor_sync(0xffffffffu, b, 16);
+        if (grp < NA && g == 0) atomicAdd(db + grp * 8 + r, b);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS));
+  }
+}
+
 // Weight and bias gradients of a 3x3 layer on the tensor cores:
 // dW[o][k] = sum_p dy[o][p] X[k][p] over the batch's pixels p (X the im2col
 // of the layer's input, k = tap * cin + ci): an M = 128 (rows o < cout, the
@@ -1451,6 +1649,27 @@ static int forward(orbit_denoiser_t* d, int nb, cudaStream_t st, bool infer = fa
   return ORBIT_OK;
 }
 
+// The row kernel of a layer's weight gradient, or none where its groups of
+// channels or pixels do not divide the layer (the first layer's one channel,
+// images of 12 x 12).
+static const int kWgRowSmem = kTcStageA + 96 * kTcKC * 4 + 1024;
+struct WgradRow {
+  void (*fn)(const float*, int, const float*, int, int, int, int, float*, float*, int*, TcWait) = nullptr;
+  int ci = 0;
+};
+static WgradRow wgrad_row_kernel(int cin, int cout, int h, int w) {
+  WgradRow k;
+  if (cin % 16 != 0 || (h * w) % kTcKC != 0 || w % 4 != 0) return k;
+  k.ci = cin % 32 == 0 ? 32 : 16;
+  if (k.ci == 32)
+    k.fn = cout == 16 ? k_conv3_wgrad_row<32, 16> : cout == 32 ? k_conv3_wgrad_row<32, 32>
+           : cout == 64 ? k_conv3_wgrad_row<32, 64> : nullptr;
+  else
+    k.fn = cout == 16 ? k_conv3_wgrad_row<16, 16> : cout == 32 ? k_conv3_wgrad_row<16, 32>
+           : cout == 64 ? k_conv3_wgrad_row<16, 64> : nullptr;
+  return k;
+}
+
 // Backward of one 3x3 layer: grad[out] holds dL/d(output after ReLU); it
 // becomes dL/d(pre-activation), the weight and bias gradients accumulate,
 // and the data gradient is written to grad[in] (no 3x3 layer's input has a
@@ -1472,9 +1691,19 @@ static int conv_bwd(orbit_denoiser_t* d, const Step3& s, int nb, cudaStream_t st
     const int spc = (stages + want - 1) / want;
     const int slices = (stages + spc - 1) / spc;
     const TcWait tw = {d->tc_wait_cycles, d->tc_withhold};
-    k_conv3_wgrad_tc<<<dim3(chunks, slices), 128, kTcSmem, st>>>(d->act[s.in], cv.cin, d->grad[s.out], cv.cout, h,
-                                                                w, nb, spc, d->d_g + cv.w_off, d->d_g + cv.b_off,
-                                                                d->d_err, tw);
+    const auto row = wgrad_row_kernel(cv.cin, cv.cout, h, w);
+    if (row.fn) {
+      const int rchunks = 3 * (cv.cin / row.ci);
+      int rwant = 4 * num_sms() / rchunks;
+      rwant = rwant < 1 ? 1 : rwant;
+      const int rspc = (stages + rwant - 1) / rwant;
+      row.fn<<<dim3(rchunks, (stages + rspc - 1) / rspc), 128, kWgRowSmem, st>>>(
+          d->act[s.in], cv.cin, d->grad[s.out], h, w, nb, rspc, d->d_g + cv.w_off, d->d_g + cv.b_off, d->d_err, tw);
+    } else {
+      k_conv3_wgrad_tc<<<dim3(chunks, slices), 128, kTcSmem, st>>>(d->act[s.in], cv.cin, d->grad[s.out], cv.cout, h,
+                                                                  w, nb, spc, d->d_g + cv.w_off, d->d_g + cv.b_off,
+                                                                  d->d_err, tw);
+    }
   } else {
     const int ttot = tiles * nb;
     const int split = ttot < 64 ? ttot : 64;
