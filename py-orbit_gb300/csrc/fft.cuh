@@ -179,6 +179,63 @@ __device__ __forceinline__ typename CT<T>::t* block_fft_fixed(typename CT<T>::t*
   return a;
 }
 
+// Lengths that are no power of two, FP64: radix-2 stages while twos are left
+// (the plan has them first), then each odd radix p with one output per thread:
+// the twiddle of input q and output r is one table entry, so an output takes
+// p - 1 complex multiply-adds, and all N outputs share the FP64 pipes.  With one
+// butterfly per thread (block_fft's general stage) the radix-5 stage of 160
+// points kept one warp busy with 136 instructions of 64 clocks: a
+// kick on 96 x 80 (192 and 160 points) 131 -> 107 us.
+template <bool INV>
+__device__ double2* block_fft_odd(double2* a, double2* b, const FftPlan& pl, const double2* __restrict__ tw) {
+  const int N = pl.n;
+  int L = 1;
+  auto next = [&]() {
+    __syncthreads();
+    double2* t = a;
+    a = b;
+    b = t;
+  };
+  for (int s = 0; s < pl.nst; ++s) {
+    const int p = pl.rad[s];
+    if (p == 2 || p == 4) {  // L is a power of two here
+      for (int h = 2; h <= p; h *= 2) {
+        const int H2 = N / 2, tws = N / (2 * L);
+        for (int t = threadIdx.x; t < H2; t += blockDim.x) {
+          const int j = t & (L - 1);
+          double2* out = b + 2 * t - j;
+          double2 w = tw[j * tws];
+          if (INV) w.y = -w.y;
+          bfly2_tw(a[t], a[t + H2], w, out[0], out[L]);
+        }
+        next();
+        L *= 2;
+      }
+      continue;
+    }
+    const int Np = N / p, tws = N / (L * p);
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+      const int r = i / Np, t = i - r * Np, j = t % L;
+      int d = j * tws + r * Np, e = 0;  // W^(q j tws) W_p^(q r)
+      if (d >= N) d -= N;
+      double2 acc = a[t];
+      for (int q = 1; q < p; ++q) {
+        e += d;
+        if (e >= N) e -= N;
+        const double2 x = a[t + q * Np];
+        double2 w = tw[e];
+        if (INV) w.y = -w.y;
+        acc.x = __fma_rn(x.x, w.x, __fma_rn(-x.y, w.y, acc.x));
+        acc.y = __fma_rn(x.x, w.y, __fma_rn(x.y, w.x, acc.y));
+      }
+      b[(t - j) * p + j + r * L] = acc;
+    }
+    next();
+    L *= p;
+  }
+  return a;
+}
+
 // a: input buffer, b: scratch, tw: the W_N table (shared memory); returns
 // the buffer holding the result.  `inv` selects the backward (+i)
 // transform; unnormalised.
@@ -187,6 +244,7 @@ __device__ typename CT<T>::t* block_fft(typename CT<T>::t* a, typename CT<T>::t*
                                         const typename CT<T>::t* __restrict__ tw, bool inv) {
   typedef typename CT<T>::t C;
   if (pl.pow2) return inv ? block_fft_pow2<T, true>(a, b, pl, tw) : block_fft_pow2<T, false>(a, b, pl, tw);
+  if constexpr (sizeof(T) == 8) return inv ? block_fft_odd<true>(a, b, pl, tw) : block_fft_odd<false>(a, b, pl, tw);
   const int N = pl.n;
   int L = 1;
   for (int s = 0; s < pl.nst; ++s) {

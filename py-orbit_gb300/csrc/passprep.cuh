@@ -82,7 +82,7 @@ static __device__ __noinline__ void prep_pass(const PrepJob& J, const ScState* s
     if (lane == 0 && ok) {
       f->n = nops;
       f->s = s;
-      f->check = x0 < xm || p0 < pm || d0 < dm;
+      f->check = !(x0 >= xm && p0 >= pm && d0 >= dm);  // (NaN among them, too)
       f->limx = __double2hiint((double)x0);
       f->limp = __double2hiint((double)p0);
       f->limd = __double2hiint((double)d0);

@@ -34,35 +34,6 @@ static const int kPassSmem = 220 * 1024;
 #define ORBIT_FX_THREADS 640
 #endif
 
-// Copies n elements of global memory (written by an earlier kernel) into
-// shared memory with asynchronous 16-byte copies (cp.async.cg: no
-// registers held, every copy of the thread in flight at once), then applies
-// f in place to the elements this thread copied, once they have landed
-// (cp.async.wait_all waits for the thread's own copies).  Threads t0.. of
-// the block take part.  Where either address is not 16-byte aligned the
-// thread copies element by element instead.  Returns with this thread's
-// elements final; the caller synchronises the block.
-template <typename T, typename F>
-__device__ __forceinline__ void copy_smem_async(T* s, const T* g, int n, F f, int t0) {
-  const int t = (int)threadIdx.x - t0, nt = (int)blockDim.x - t0;
-  if (t < 0) return;
-  constexpr int E = 16 / (int)sizeof(T);  // elements per 16-byte copy
-  const uint32_t sb = (uint32_t)__cvta_generic_to_shared(s);
-  const bool aligned = ((sb | (uint32_t)(size_t)g) & 15u) == 0u;
-  const int nb = aligned ? n / E : 0;
-  for (int i = t; i < nb; i += nt)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sb + 16u * (uint32_t)i),
-                 "l"(reinterpret_cast<const char*>(g) + 16 * (size_t)i)
-                 : "memory");
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  for (int i = t; i < nb; i += nt) {
-#pragma unroll
-    for (int q = 0; q < E; ++q) s[i * E + q] = f(s[i * E + q]);
-  }
-  for (int i = nb * E + t; i < n; i += nt) s[i] = f(__ldcg(g + i));
-}
-
 // The kick constants of a pass (one thread), out of line so that their
 // registers do not weigh on the particle loop's.
 __device__ __noinline__ void kick_consts_into(KickConst* k, KickFix* kf, const KickArgs& kick) {
@@ -158,6 +129,7 @@ __device__ __noinline__ void pass_particle(FxFallback* f, int i, bool first) {
     ExtAcc e;
     e.init();
     e.add(p.x, p.y, p.z);
+    e.finish();
     for (int c = 0; c < 3; ++c) {
       atomicMin(&f->mn[c], e.mn[c]);
       atomicMax(&f->mx[c], e.mx[c]);
@@ -369,7 +341,7 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
     ext.init();
     mag.init();
   }
-  for (int i = blk * blockDim.x + threadIdx.x; i < n; i += nblk * blockDim.x) {
+  for (int i = first_particle(blk, nblk); i < n; i += nblk * blockDim.x) {
     bool ok = fixed;
     fx::Part t;
     if (ok) {

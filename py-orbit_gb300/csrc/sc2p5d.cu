@@ -22,6 +22,9 @@ static const int kMaxSmem = 220 * 1024;
 #ifndef ORBIT_DEP_THREADS
 #define ORBIT_DEP_THREADS 1024
 #endif
+#ifndef ORBIT_KICK_THREADS
+#define ORBIT_KICK_THREADS 640
+#endif
 #ifndef ORBIT_MIN_THREADS
 #define ORBIT_MIN_THREADS 256
 #endif
@@ -52,12 +55,28 @@ double sc_rb_long_factor(const orbit_sync_t& s, double length) {
 // ---------------------------------------------------------------------
 // Extrema scan; the last block sets up the grids for the kick.  The
 // accumulation grids start at zero: the kernels that read them clear them.
+// Bound by the latency of its loads and of the set-up (24 MB for 1e6 particles
+// are 4 us): four particles' loads in flight a thread.  A whole
+// kick of 1e6 particles in a pipe 172 -> 160 us, of 2e6 with RB 278 -> 253.
 __global__ void k_extrema(const double* __restrict__ x, const double* __restrict__ y,
                           const double* __restrict__ z, int n, ScState* st, unsigned* status,
                           const __grid_constant__ SetupArgs sa) {
   ExtAcc a;
   a.init();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a.add(x[i], y[i], z[i]);
+  const int di = gridDim.x * blockDim.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i < n - 3 * di; i += 4 * di) {
+    double v[4][3];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k][0] = x[i + k * di];
+      v[k][1] = y[i + k * di];
+      v[k][2] = z[i + k * di];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a.add(v[k][0], v[k][1], v[k][2]);
+  }
+  for (; i < n; i += di) a.add(x[i], y[i], z[i]);
   ext_commit_and_setup(a, st, status, sa, gridDim.x);
 }
 
@@ -619,17 +638,23 @@ __device__ double rb_deriv_cell(const double* lam, int nz, int navg, double zmin
   return __ddiv_rn(y, dz);
 }
 
-// 2.5Drb analysis on the finished grids (one block): the rho-grid moments
+// 2.5Drb analysis on the finished grids: the rho-grid moments
 // that give the beam centre and a_bunch = sqrt(2 (<x^2> + <y^2>))
 // (SpaceChargeCalc2p5Drb.cc:226-254; the reference takes y from the x grid,
 // kept), the total macrosize the kick divides by, the pipe-radius terms of
 // the longitudinal kick (:124-136) and the derivative grid.
+// Blocks of the grid's rows sum the moments, the last to finish adds the blocks'
+// sums in their order; the derivative cells go round the blocks.  One block for
+// all of it took 79 us on 128 x 128 x 64, this 19.
+static const int kRbBlocks = 64;
+
 __global__ void k_rb_analysis(ScState* st, const double* __restrict__ rho, const double* __restrict__ lam,
-                              double* lamd, int nx, int ny, int nz, int navg, double pipe_radius) {
+                              double* lamd, int nx, int ny, int nz, int navg, double pipe_radius,
+                              double* __restrict__ parts, unsigned* count) {
   if (st->skip) return;
   const double xmin = st->xmin, dx = st->dx;
   double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int idx = threadIdx.x; idx < nx * ny; idx += blockDim.x) {
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nx * ny; idx += gridDim.x * blockDim.x) {
     int ix = idx / ny, iy = idx - ix * ny;
     double val = rho[idx];
     double x = __dadd_rn(xmin, __dmul_rn((double)ix, dx));
@@ -646,27 +671,39 @@ __global__ void k_rb_analysis(ScState* st, const double* __restrict__ rho, const
   if ((threadIdx.x & 31) == 0)
     for (int c = 0; c < 5; ++c) red[threadIdx.x >> 5][c] = s[c];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
-      for (int c = 0; c < 5; ++c) t[c] += red[w][c];
-    double total = t[0];
-    double xa = t[1] / total, x2 = t[2] / total, ya = t[3] / total, y2 = t[4] / total;
-    x2 = fabs(x2 - xa * xa);
-    y2 = fabs(y2 - ya * ya);
-    double a = sqrt(2 * (x2 + y2));
-    st->rb_xc = xa;
-    st->rb_yc = ya;
-    st->rb_a2 = a * a;
-    st->rb_lin = 1.0 + 2 * log(pipe_radius / a);
-    st->rb_lout = 2 * log(pipe_radius);
-    st->total_m = total;
+  if (threadIdx.x < 5) {
+    double t = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w][threadIdx.x];
+    parts[5 * blockIdx.x + threadIdx.x] = t;
+  }
+  if (last_block_done(count, gridDim.x) && threadIdx.x < 32) {
+    const int lane = threadIdx.x, c = lane < 5 ? lane : 0;
+    double t = 0.0;
+    for (int b = 0; b < (int)gridDim.x; ++b) t += __ldcg(parts + 5 * b + c);
+    const double total = __shfl_sync(0xffffffffu, t, 0);
+    t = t / total;
+    const double xa = __shfl_sync(0xffffffffu, t, 1), ya = __shfl_sync(0xffffffffu, t, 3);
+    const double x2 = fabs(__shfl_sync(0xffffffffu, t, 2) - xa * xa);
+    const double y2 = fabs(__shfl_sync(0xffffffffu, t, 4) - ya * ya);
+    const double a = sqrt(2 * (x2 + y2));
+    const double q = (lane == 0 ? pipe_radius : 1.0) / (lane == 0 ? a : a * a);  // lane 1: 1 / a^2
+    const double lg = log(lane == 0 ? q : pipe_radius);
+    if (lane == 0) {
+      st->rb_xc = xa;
+      st->rb_yc = ya;
+      st->rb_a2 = a * a;
+      st->rb_lin = 1.0 + 2 * lg;
+      st->total_m = total;
+    } else if (lane == 1) {
+      st->rb_inv_a2 = q;
+      st->rb_lout = 2 * lg;
+    }
   }
   const double zmin = st->zmin, dz = st->dz;
   if (nz == 1) {
-    if (threadIdx.x == 0) lamd[0] = 0.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) lamd[0] = 0.0;
   } else if (nz == 2) {
-    if (threadIdx.x == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
       // Grid1D::calcGradient at the midpoint (Grid1D.cc:520-534, 568-627)
       double g0 = __dadd_rn(zmin, __dmul_rn(0.5, dz)), g1 = __dadd_rn(zmin, __dmul_rn(1.5, dz));
       double zm = __dmul_rn(__dadd_rn(g0, g1), 0.5);
@@ -685,7 +722,7 @@ __global__ void k_rb_analysis(ScState* st, const double* __restrict__ rho, const
       lamd[1] = __ddiv_rn(d, dz);
     }
   } else {
-    for (int iz = threadIdx.x; iz < nz; iz += blockDim.x) lamd[iz] = rb_deriv_cell(lam, nz, navg, zmin, dz, iz);
+    for (int iz = threadIdx.x * gridDim.x + blockIdx.x; iz < nz; iz += gridDim.x * blockDim.x) lamd[iz] = rb_deriv_cell(lam, nz, navg, zmin, dz, iz);
   }
 }
 
@@ -808,42 +845,68 @@ __global__ void __launch_bounds__(768) k_deposit_band(const double* __restrict__
 }
 
 // Kick (SpaceChargeCalc2p5D.cc:104-119): fixed-point gradient and line
-// density (kick_fixed), FP64 routine for the particles it declines.  With
-// lamd (2.5Drb) also the longitudinal kick of dE.
-template <bool SMEM>
-__global__ void k_kick_plain(const double* __restrict__ x, double* __restrict__ xp, const double* __restrict__ y,
+// density (kick_direct), FP64 routine for the particles it declines.  RB: the
+// longitudinal kick of dE besides.
+//
+// Bound by instruction issue, with the FP64 pipe (14 conversions and multiply-
+// Bound by instruction issue, with the FP64 pipe (14 conversions and multiply-
+// adds a particle, 28 with RB) close behind.  128 x 128 x 64: 1e6 particles in a
+// pipe 75 -> 48 us; 2e6 with RB, where a division and a logarithm held the FP64
+// pipe, 290 -> 112 us.  512, 640 and 768 threads are within 1%.
+template <bool SMEM, bool RB>
+__global__ void __launch_bounds__(ORBIT_KICK_THREADS) k_kick_plain(const double* __restrict__ x, double* __restrict__ xp, const double* __restrict__ y,
                              double* __restrict__ yp, const double* __restrict__ z, int n, const ScState* st,
                              const double* __restrict__ phi, const double* __restrict__ lam,
                              const long long* __restrict__ phi_fix, const long long* __restrict__ lam_fix,
                              double host_factor, int nx, int ny, int nz, const double* __restrict__ lamd,
-                             double rb_lsf, double* __restrict__ dE, BndShape bnd) {
-  KickConst k;
-  KickFix kf;
-  load_kick_block(k, &kf, st, host_factor, nx, ny, nz);
-  if (k.skip) return;
-  extern __shared__ long long s_phix[];
-  const long long* P = phi_fix;
-  const long long* Lm = lam_fix;
-  if (SMEM) {
-    // the shared copy is converted here; phi_fix, lam_fix are not read
-    for (int i = threadIdx.x; i < nx * ny; i += blockDim.x) s_phix[i] = fx_pair(phi_fixed(phi[i], kf.sphi));
-    for (int i = threadIdx.x; i < nz; i += blockDim.x) s_phix[nx * ny + i] = fx_pair(phi_fixed(lam[i], kf.slam));
-    __syncthreads();
-    P = s_phix;
-    Lm = s_phix + nx * ny;
+                             double rb_lsf, const LogTab* __restrict__ log_tab, double* __restrict__ dE,
+                             BndShape bnd) {
+  if (st->skip) return;
+  __shared__ KickConst s_k;
+  __shared__ KickFix s_kf;
+  __shared__ KickDirect s_d;
+  __shared__ LogTab s_log;
+  extern __shared__ __align__(16) long long s_phix[];
+  const long long* P = SMEM ? s_phix : phi_fix;
+  const long long* Lm = SMEM ? s_phix + nx * ny : lam_fix;
+  // warp 0 makes the constants while the others fill the block's copy of the
+  // potential (phi_fix, lam_fix are not read then)
+  if (threadIdx.x < 32) {
+    if (threadIdx.x < 3) load_kick_direct(&s_d, st, nx, ny, nz);
+    if (threadIdx.x == 0) {
+      load_kick_const(s_k, st, host_factor, nx, ny, nz, false);
+      load_kick_fix(s_kf, st, s_k.fac, nx, ny, nz);
+      s_d.gxs = s_kf.gxs; s_d.gys = s_kf.gys; s_d.lfs = s_kf.lfs;
+    }
   }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  if (SMEM) {
+    const int sphi = scale_bits(st->phi_absmax), slam = scale_bits(st->lam_absmax);
+    double* sd = reinterpret_cast<double*>(s_phix);
+    copy_smem_async(sd, phi, nx * ny, [sphi](double v) { return __longlong_as_double(fx_pair(phi_fixed(v, sphi))); }, 32);
+    copy_smem_async(sd + nx * ny, lam, nz,
+                    [slam](double v) { return __longlong_as_double(fx_pair(phi_fixed(v, slam))); }, 32);
+  }
+  if (RB)
+    for (int i = threadIdx.x; i < (int)(sizeof(LogTab) / 4); i += blockDim.x)
+      reinterpret_cast<unsigned*>(&s_log)[i] = reinterpret_cast<const unsigned*>(log_tab)[i];
+  __syncthreads();
+  const KickDirect d = s_d;
+  RbConst r;
+  if (RB) load_rb_const(r, st, rb_lsf);
+  for (int i = first_particle(blockIdx.x, gridDim.x); i < n; i += gridDim.x * blockDim.x) {
     double a = xp[i], b = yp[i];
-    double xi = x[i], yi = y[i], zi = z[i];
+    const double xi = x[i], yi = y[i], zi = z[i];
     if (!bnd_inside(bnd, xi, yi)) continue;  // SpaceChargeCalc2p5D.cc:110
-    if (!kick_fixed(kf, P, Lm, xi, yi, zi, a, b)) kick_plain(k, phi, lam, xi, yi, zi, a, b);
+    int iz;
+    long long w;
+    const bool ok = kick_direct(d, P, Lm, nx, ny, nz, xi, yi, zi, a, b, iz, w);
+    if (!ok) kick_plain(s_k, phi, lam, xi, yi, zi, a, b);
     xp[i] = a;
     yp[i] = b;
-    if (lamd) {
-      RbConst r;
-      load_rb_const(r, st, rb_lsf);
+    if (RB) {
       double e = dE[i];
-      kick_rb_long(k, r, lamd, xi, yi, zi, e);
+      if (ok) kick_rb_direct(r, &s_log, lamd, nz, xi, yi, iz, w, e);
+      else kick_rb_long(s_k, r, lamd, xi, yi, zi, e);
       dE[i] = e;
     }
   }
@@ -1140,7 +1203,7 @@ static int set_fft_attrs(int nmax) {
 
 static int ext_blocks(int n) {
   int b = (n + 255) / 256;
-  int cap = num_sms() * 4;
+  int cap = num_sms() * 2;
   return b < 1 ? 1 : (b > cap ? cap : b);
 }
 
@@ -1499,9 +1562,10 @@ static int max_threads_of(K kernel) {
 // plain (shared, global), kick fp32 (shared, global).  Queried once,
 // outside any stream capture (init_attrs).
 static const int* particle_kernel_threads() {
-  static const int mt[6] = {max_threads_of(k_deposit_plain<true>), max_threads_of(k_deposit_plain<false>),
-                            max_threads_of(k_kick_plain<true>), max_threads_of(k_kick_plain<false>),
-                            max_threads_of(k_kick_fp32<true>), max_threads_of(k_kick_fp32<false>)};
+  static const int mt[8] = {max_threads_of(k_deposit_plain<true>), max_threads_of(k_deposit_plain<false>),
+                            max_threads_of(k_kick_plain<true, true>), max_threads_of(k_kick_plain<false, true>),
+                            max_threads_of(k_kick_fp32<true>), max_threads_of(k_kick_fp32<false>),
+                            max_threads_of(k_kick_plain<true, false>), max_threads_of(k_kick_plain<false, false>)};
   return mt;
 }
 
@@ -1747,8 +1811,8 @@ int sc_enqueue_kick(orbit_sc2p5d_t* c, orbit_bunch_t* b, double length, cudaStre
   if (c->rb) {
     // beam centre, a_bunch and the derivative grid from the finished grids
     ORBIT_PB("rb_analysis", s);
-    k_rb_analysis<<<1, 512, 0, s>>>(c->d_st, c->d_rho, c->d_lam, c->d_lamd, c->nx, c->ny, c->nz, c->n_long_avg,
-                                     pipe_radius);
+    k_rb_analysis<<<kRbBlocks, 256, 0, s>>>(c->d_st, c->d_rho, c->d_lam, c->d_lamd, c->nx, c->ny, c->nz,
+                                            c->n_long_avg, pipe_radius, c->d_rb_parts, c->d_rb_count);
     ORBIT_PE(s);
     ++nl;
     ORBIT_LAUNCH_CHECK("sc2p5drb analysis");
@@ -1794,21 +1858,16 @@ int sc_enqueue_kick(orbit_sc2p5d_t* c, orbit_bunch_t* b, double length, cudaStre
     double lsf = c->rb ? sc_rb_long_factor(b->sync, length) : 0.0;
     BndShape bshape = bnd_shape_of(bnd);
     size_t smk = (plain ? sizeof(double) : sizeof(float)) * ((size_t)c->nx * c->ny + c->nz);
-    const int* mt_kick = particle_kernel_threads() + 2;
-    particle_geometry(c->smem_kick ? smk : 0, n, mt_kick[(plain ? 0 : 2) + (c->smem_kick ? 0 : 1)], false,
-                      &blocks, &threads);
+    const int* mt_kick = particle_kernel_threads() + (plain ? (c->rb ? 2 : 6) : 4);
+    particle_geometry(c->smem_kick ? smk : 0, n, mt_kick[c->smem_kick ? 0 : 1], false, &blocks, &threads);
     ORBIT_PB("kick", s);
     if (plain) {
-      if (c->smem_kick)
-        k_kick_plain<true><<<blocks, threads, smk, s>>>(b->coord(0), b->coord(1), b->coord(2), b->coord(3),
-                                                        b->coord(4), n, c->d_st, c->d_phi, c->d_lam, c->d_phi_fix,
-                                                        c->d_lam_fix, hf, c->nx, c->ny, c->nz, lamd, lsf,
-                                                        b->coord(5), bshape);
-      else
-        k_kick_plain<false><<<blocks, threads, 0, s>>>(b->coord(0), b->coord(1), b->coord(2), b->coord(3),
+      auto* k = c->smem_kick ? (c->rb ? k_kick_plain<true, true> : k_kick_plain<true, false>)
+                             : (c->rb ? k_kick_plain<false, true> : k_kick_plain<false, false>);
+      k<<<blocks, threads, c->smem_kick ? smk : 0, s>>>(b->coord(0), b->coord(1), b->coord(2), b->coord(3),
                                                        b->coord(4), n, c->d_st, c->d_phi, c->d_lam, c->d_phi_fix,
                                                        c->d_lam_fix, hf, c->nx, c->ny, c->nz, lamd, lsf,
-                                                       b->coord(5), bshape);
+                                                       c->d_log_tab, b->coord(5), bshape);
     } else {
       if (c->smem_kick)
         k_kick_fp32<true><<<blocks, threads, smk, s>>>(b->coord(0), b->coord(1), b->coord(2), b->coord(3),
@@ -1852,8 +1911,10 @@ static int init_attrs(orbit_sc2p5d_t* c) {
   if (c->smem_deposit && dep > 48 * 1024)
     ORBIT_CUDA(cudaFuncSetAttribute(k_deposit_plain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
   if (c->form == ORBIT_FORM_PLAIN) {
-    if (c->smem_kick && kick > 48 * 1024)
-      ORBIT_CUDA(cudaFuncSetAttribute(k_kick_plain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+    if (c->smem_kick && kick > 48 * 1024) {
+      ORBIT_CUDA(cudaFuncSetAttribute(k_kick_plain<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+      ORBIT_CUDA(cudaFuncSetAttribute(k_kick_plain<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+    }
     int nmax = c->nx2 > c->ny2 ? c->nx2 : c->ny2;
     int rc = set_fft_attrs<double>(nmax);
     return rc ? rc : init_conv_fused<double>(c);
@@ -1964,6 +2025,7 @@ int orbit_sc2p5d_destroy(orbit_sc2p5d_t* c) {
   if (c->done) cudaEventDestroy(c->done);
   if (c->aux) cudaStreamDestroy(c->aux);
   void* ptrs[] = {c->d_st, c->d_prep, c->d_rho_q, c->d_z_q, c->d_rho, c->d_phi, c->d_lam, c->d_lamd,
+                  c->d_rb_parts, c->d_rb_count, c->d_log_tab,
                   c->d_phi_f, c->d_lam_f, c->d_hat, c->d_green, c->d_gbuf, c->d_gscratch, c->d_tw_x, c->d_tw_y,
                   c->d_phi_fix, c->d_lam_fix, c->d_dn_parts, c->d_dn_raw, c->d_dn_hat, c->d_dn_phi,
                   c->d_dn_st};
@@ -2054,6 +2116,18 @@ int orbit_sc2p5d_track_boundary(orbit_sc2p5d_t* c, orbit_bunch_t* b, double leng
 int orbit_sc2p5drb_create(orbit_sc2p5d_t** out, int nx, int ny, int nz, double xy_ratio) {
   int rc = orbit_sc2p5d_create(out, nx, ny, nz, xy_ratio, ORBIT_FORM_PLAIN);
   if (rc) return rc;
+  LogTab t;
+  make_log_tab(&t);
+  cudaError_t e = cudaMalloc((void**)&(*out)->d_rb_parts, sizeof(double) * 5 * kRbBlocks);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&(*out)->d_rb_count, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset((*out)->d_rb_count, 0, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&(*out)->d_log_tab, sizeof(LogTab));
+  if (e == cudaSuccess) e = cudaMemcpy((*out)->d_log_tab, &t, sizeof(t), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    orbit_sc2p5d_destroy(*out);
+    *out = nullptr;
+    return cuda_error(e, "orbit_sc2p5drb_create");
+  }
   (*out)->rb = true;
   (*out)->n_long_avg = 3;  // SpaceChargeCalc2p5Drb.cc:42
   return ORBIT_OK;

@@ -30,7 +30,7 @@ struct ScState {
   unsigned ext_count;                                     // blocks done with the extrema scan (last one sets up)
   // 2.5Drb: beam centre, a_bunch^2 and the two pipe-radius terms of the
   // longitudinal kick (SpaceChargeCalc2p5Drb.cc:124-136, 226-254)
-  double rb_xc, rb_yc, rb_a2, rb_lin, rb_lout;
+  double rb_xc, rb_yc, rb_a2, rb_inv_a2, rb_lin, rb_lout;
   unsigned long long n_kicks, n_green;                    // kicks solved, Green spectra rebuilt
   // learned closure: fallen back to the plain deposit (sticky), the last
   // check's relative rms potential difference, checks and fall-backs
@@ -110,6 +110,7 @@ struct orbit_denoiser;
 namespace orbit {
 struct DevOp;
 struct PassPrep;
+struct LogTab;
 // The lattice pass that follows a kick, for the constants made beside its
 // solve (prep_pass): maps ops[a..b), dp_p per dE and the kick factor; out
 // null: none.
@@ -182,6 +183,9 @@ struct orbit_sc2p5d {
   bool rb = false;
   int n_long_avg = 3;
   double* d_lamd = nullptr;               // derivative grid (nz)
+  double* d_rb_parts = nullptr;           // the analysis's per-block sums, and its block counter
+  unsigned* d_rb_count = nullptr;
+  orbit::LogTab* d_log_tab = nullptr;
   int dep_threads = 512, kick_threads = 512;
   // learned closure (both forms): the network, the check period and bound,
   // the host kick counter, and the output-sum, raw-density and check-solve
