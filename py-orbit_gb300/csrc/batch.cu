@@ -164,6 +164,27 @@ static int wave_chunk(const orbit_batch_t* bt, const BatchClass& c, int waves, i
   return lo;
 }
 
+// The class's candidate shapes at the members' present sizes.
+static void fill_candidates(const orbit_batch_t* bt, BatchClass& c) {
+  const int bands = batch_deposit_bands(c.proto);
+  for (int q = 0; q < kMaxDep; ++q) {
+    c.dep_cand[q][0] = kDepCand[q < kNDep ? q : 0][0];
+    c.dep_cand[q][1] = q < kNDep ? kDepCand[q][1] : wave_chunk(bt, c, 1 + q - kNDep, bands);
+  }
+  for (int q = 0; q < kMaxPass; ++q) {
+    c.pass_cand[q][0] = ORBIT_PASS_THREADS;
+    c.pass_cand[q][1] = q < kNPass ? kPassCand[q][1] : wave_chunk(bt, c, 1 + q - kNPass, 1);
+  }
+}
+
+// The chosen shapes as orbit_batch_class reports them.
+static void report_shapes(BatchClass& c) {
+  c.tune.dep_threads = c.dep_cand[c.dep_sel][0];
+  c.tune.dep_chunk = c.dep_cand[c.dep_sel][1];
+  c.tune.pass_threads = c.pass_cand[c.pass_sel][0];
+  c.tune.pass_chunk = c.pass_cand[c.pass_sel][1];
+}
+
 // Blocks of each member for `chunk` particles per `per` blocks.
 static int build_map(const orbit_batch_t* bt, const BatchClass& c, int chunk, int per, BlockMap& out) {
   std::vector<unsigned short> bj;
@@ -256,17 +277,10 @@ static int build_tables(orbit_batch_t* bt, BatchClass& c) {
   if (rc) return rc;
   c.dep_maps.resize(kMaxDep);
   c.pass_maps.resize(kMaxPass);
+  fill_candidates(bt, c);
   const int bands = batch_deposit_bands(c.proto);
-  for (int q = 0; q < kMaxDep && !rc; ++q) {
-    c.dep_cand[q][0] = q < kNDep ? kDepCand[q][0] : kDepCand[0][0];
-    c.dep_cand[q][1] = q < kNDep ? kDepCand[q][1] : wave_chunk(bt, c, 1 + q - kNDep, bands);
-    rc = build_map(bt, c, c.dep_cand[q][1], bands, c.dep_maps[q]);
-  }
-  for (int q = 0; q < kMaxPass && !rc; ++q) {
-    c.pass_cand[q][0] = ORBIT_PASS_THREADS;
-    c.pass_cand[q][1] = q < kNPass ? kPassCand[q][1] : wave_chunk(bt, c, 1 + q - kNPass, 1);
-    rc = build_map(bt, c, c.pass_cand[q][1], 1, c.pass_maps[q]);
-  }
+  for (int q = 0; q < kMaxDep && !rc; ++q) rc = build_map(bt, c, c.dep_cand[q][1], bands, c.dep_maps[q]);
+  for (int q = 0; q < kMaxPass && !rc; ++q) rc = build_map(bt, c, c.pass_cand[q][1], 1, c.pass_maps[q]);
   return rc;
 }
 
@@ -300,10 +314,16 @@ static int compile_all(orbit_batch_t* bt) {
     if (!ok) return set_error(ORBIT_ERR_ARG, "orbit_batch: the members' lattices differ in structure");
   }
   bt->plan = plans[0];
+  // one launch serves all members: fixed point where every member's maps have that form (poles and charges differ)
+  for (size_t m = 1; m < nmem; ++m) {
+    for (size_t i = 0; i < bt->plan.segs.size(); ++i) bt->plan.segs[i].fx = bt->plan.segs[i].fx && plans[m].segs[i].fx;
+    bt->plan.wrap.fx = bt->plan.wrap.fx && plans[m].wrap.fx;
+  }
   bt->nsc = (int)bt->plan.sc_idx.size();
   for (auto& c : bt->classes) {
     int rc = build_tables(bt, c);
     if (rc) return rc;
+    if (bt->tuned) report_shapes(c);  // the wave shapes follow the bunch sizes
   }
   bt->key_n.resize(nmem);
   bt->key_ms.resize(nmem);
@@ -493,14 +513,6 @@ static int probe_fft(orbit_batch_t* bt) {
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   return rc;
-}
-
-// The chosen shapes as orbit_batch_class reports them.
-static void report_shapes(BatchClass& c) {
-  c.tune.dep_threads = c.dep_cand[c.dep_sel][0];
-  c.tune.dep_chunk = c.dep_cand[c.dep_sel][1];
-  c.tune.pass_threads = c.pass_cand[c.pass_sel][0];
-  c.tune.pass_chunk = c.pass_cand[c.pass_sel][1];
 }
 
 // Median time of each candidate shape over the tuning turn; the fastest
@@ -781,12 +793,12 @@ int orbit_batch_set_tuning(orbit_batch_t* bt, int cls, const int* tuning) {
     return set_error(ORBIT_ERR_ARG, "orbit_batch_set_tuning: bad argument");
   BatchClass& c = bt->classes[cls];
   int ds = -1, ps = -1;
-  // the class's own shapes are known once it is compiled
+  if (!bt->compiled) fill_candidates(bt, c);  // a shape reported by another batch of the same bunches
   auto is = [](const int cand[2], int threads, int chunk) { return cand[0] == threads && cand[1] == chunk; };
   for (int q = kMaxDep - 1; q >= 0; --q)
-    if (is(q < kNDep ? kDepCand[q] : c.dep_cand[q], tuning[0], tuning[1])) ds = q;
+    if (is(c.dep_cand[q], tuning[0], tuning[1])) ds = q;
   for (int q = kMaxPass - 1; q >= 0; --q)
-    if (is(q < kNPass ? kPassCand[q] : c.pass_cand[q], tuning[2], tuning[3])) ps = q;
+    if (is(c.pass_cand[q], tuning[2], tuning[3])) ps = q;
   if (ds < 0 || ps < 0 || (tuning[4] != 0 && tuning[4] != 1))
     return set_error(ORBIT_ERR_ARG, "orbit_batch_set_tuning: not one of the candidate shapes");
   if (bt->used) ORBIT_CUDA(cudaStreamSynchronize(bt->stream));

@@ -649,9 +649,6 @@ int compile(orbit_program_t* p, orbit_bunch_t* bu, Plan& plan) {
       p->time_adv[k] = adv;
       if (d.code == ORBIT_OP_WEDGEROT || (d.code == ORBIT_OP_KICK && d.c[2] != 0.)) s.dE = true;
       if (d.code == 0) continue;
-      if (bu->sync.charge == 0. &&
-          (d.code == ORBIT_OP_MULTP || d.code == ORBIT_OP_MPFRIN || d.code == ORBIT_OP_MPFROUT))
-        continue;  // no effect on a neutral bunch (teapotbase.cc:340, 397, 510)
       if (lengthwise(d.code) && (int)dev.size() > s.a && lengthwise(dev.back().code) == lengthwise(d.code)) {
         dev.back().c[0] += d.c[0];
         continue;
@@ -682,7 +679,9 @@ int compile(orbit_program_t* p, orbit_bunch_t* bu, Plan& plan) {
     bool moves = false;
     sg.fx = sg.b - sg.a < fx::kMaxOps;
     for (int k = sg.a; k < sg.b; ++k) {
-      sg.fx = sg.fx && fx::supported(dev[k]);
+      // multipoles do nothing to a neutral bunch (teapotbase.cc:340, 397, 510): left to the FP64 routines
+      const bool pole = dev[k].code == ORBIT_OP_MULTP || dev[k].code == ORBIT_OP_MPFRIN || dev[k].code == ORBIT_OP_MPFROUT;
+      sg.fx = sg.fx && fx::supported(dev[k]) && !(pole && bu->sync.charge == 0.);
       moves = moves || fx::moves_x(dev[k]);
     }
     sg.fx = sg.fx && moves;  // x and y are rewritten: thin kicks alone leave them as they are
