@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 #include <cstdint>
+#include <mutex>
 #include <string>
 
 #include "../../include/orbit_gb300.h"
@@ -101,5 +102,6 @@ struct orbit_bunch {
   double* d_phase = nullptr;
   int phase_cap = 0;
   double* d_diag = nullptr;
+  std::mutex diag_mu;           // held from a moments launch until its sums are read
   double* coord(int c) const { return d_coords + (size_t)c * cap; }
 };

@@ -287,6 +287,7 @@ extern "C" {
 int orbit_bunch_moments(orbit_bunch_t* b, double* out) {
   if (!b || !out) return set_error(ORBIT_ERR_ARG, "orbit_bunch_moments: bad argument");
   const int nb = moment_blocks();
+  std::lock_guard<std::mutex> lock(b->diag_mu);
   DiagScratch d;
   int rc = diag_scratch(b, &d);
   if (rc) return rc;
@@ -317,6 +318,7 @@ int orbit_bunch_xy_moments(orbit_bunch_t* b, int order, const double* params, do
     return set_error(ORBIT_ERR_ARG, "orbit_bunch_xy_moments: bad argument (2 <= order <= 16)");
   const int nc = xy_cells(order);
   const bool uniform = !b->has_msize;
+  std::unique_lock<std::mutex> lock(b->diag_mu);
   DiagScratch d;
   int rc = diag_scratch(b, &d);
   if (rc) return rc;
@@ -340,6 +342,7 @@ int orbit_bunch_xy_moments(orbit_bunch_t* b, int order, const double* params, do
     ORBIT_CUDA(cudaMemcpyAsync(sum, d.res, sizeof(double) * nc, cudaMemcpyDeviceToHost, b->stream));
     ORBIT_CUDA(cudaStreamSynchronize(b->stream));
   }
+  lock.unlock();
   // total macrosize: n for a uniform macrosize (the reference's m_size = 1
   // there), else the sum of the macrosizes
   double total = (double)b->n;
@@ -351,12 +354,19 @@ int orbit_bunch_xy_moments(orbit_bunch_t* b, int order, const double* params, do
   }
   const int w = order + 1;
   for (int k = 0; k < w * w; ++k) out[k] = 0.0;
+  // pow(xbetaterm, double(i)) pow(ybetaterm, double(j)) (BunchTwissAnalysis.cc:249),
+  // in long double: a term's divisions average out over the bunch, the sum's would not
+  long double xb[17], yb[17];
+  xb[0] = yb[0] = 1.0L;
+  for (int i = 1; i <= order; ++i) {
+    xb[i] = xb[i - 1] * params[5];
+    yb[i] = yb[i - 1] * params[6];
+  }
   int k = 0;
   for (int j = 0; j < order; ++j)
     for (int i = 0; i < order + 1 - j; ++i, ++k) {
-      // pow(xbetaterm, double(i)) (BunchTwissAnalysis.cc:249)
-      const double t = sum[k] / std::pow(params[5], (double)i) / std::pow(params[6], (double)j);
-      out[i * w + j] += uniform ? t : t + sum[k];
+      const long double t = sum[k] / (xb[i] * yb[j]);
+      out[i * w + j] += (double)(uniform ? t : t + sum[k]);
     }
   if (uniform) out[2 * w + order] += sum[k];
   // BunchTwissAnalysis.cc:325-336: divided for i + j <= order (the stray

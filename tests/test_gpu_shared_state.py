@@ -1,10 +1,13 @@
 """State shared between bunches and calls: batches whose members differ in what
-the fixed-point pass depends on, block shapes carried from one batch to another.
+the fixed-point pass depends on, block shapes carried from one batch to another,
+and one bunch's moments asked for by two threads.
 
 Tolerance: the members of a mixed batch take the FP64 pass where single-bunch
 tracking takes the fixed-point one; 2e-11 for at most 20 kicks (half of
 1e-10 per 100 kicks, the bound coordinates are held to elsewhere, for so short a
 line)."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -58,3 +61,21 @@ def test_shapes_reported_by_one_batch_are_taken_by_a_new_one():
         fresh.trackTurns(1)
         assert [fresh.classes()[k][q] for q in keys] == [c[q] for q in keys]
 
+
+def test_moments_of_one_bunch_from_two_threads():
+    from orbit_gb300 import workloads as W
+    dev = W.make_bunch(W.c2_coords(50_000, seed=5), 1.0)._device_bunch()
+    par = [0.0, 1.9, 0.77, 1e-4, -2e-4, 2.1e-3, 1.7e-3]
+    want = {o: dev.xy_moments(o, par) for o in (2, 8)}
+    bad = []
+
+    def work(order):
+        for _ in range(40):
+            if not np.array_equal(dev.xy_moments(order, par), want[order]):
+                bad.append(order)
+    ts = [threading.Thread(target=work, args=(o,)) for o in want]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
