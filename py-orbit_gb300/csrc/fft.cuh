@@ -186,6 +186,12 @@ __device__ __forceinline__ typename CT<T>::t* block_fft_fixed(typename CT<T>::t*
 // butterfly per thread (block_fft's general stage) the radix-5 stage of 160
 // points kept one warp busy with 136 instructions of 64 clocks: a
 // kick on 96 x 80 (192 and 160 points) 131 -> 107 us.
+// Products are summed before the input that carries most of the sum is added, and a
+// radix-2 product is rounded before its two sums: one rounding of the largest
+// partial sum per output, as block_fft has it.  Error of the gradient of a
+// 1-D convolution with log r at 192 and 320 points: 1.80e-14 and 4.0e-14; 2.2e-14
+// and 5.6e-14 with the sum started from that input; 1.89e-14 and 4.5e-14 with
+// block_fft's stages.
 template <bool INV>
 __device__ double2* block_fft_odd(double2* a, double2* b, const FftPlan& pl, const double2* __restrict__ tw) {
   const int N = pl.n;
@@ -206,7 +212,9 @@ __device__ double2* block_fft_odd(double2* a, double2* b, const FftPlan& pl, con
           double2* out = b + 2 * t - j;
           double2 w = tw[j * tws];
           if (INV) w.y = -w.y;
-          bfly2_tw(a[t], a[t + H2], w, out[0], out[L]);
+          const double2 x0 = a[t], x1 = c_mul(a[t + H2], w);
+          out[0] = c_add(x0, x1);
+          out[L] = c_sub(x0, x1);
         }
         next();
         L *= 2;
@@ -218,7 +226,7 @@ __device__ double2* block_fft_odd(double2* a, double2* b, const FftPlan& pl, con
       const int r = i / Np, t = i - r * Np, j = t % L;
       int d = j * tws + r * Np, e = 0;  // W^(q j tws) W_p^(q r)
       if (d >= N) d -= N;
-      double2 acc = a[t];
+      double2 acc = make_double2(0.0, 0.0);
       for (int q = 1; q < p; ++q) {
         e += d;
         if (e >= N) e -= N;
@@ -228,6 +236,7 @@ __device__ double2* block_fft_odd(double2* a, double2* b, const FftPlan& pl, con
         acc.x = __fma_rn(x.x, w.x, __fma_rn(-x.y, w.y, acc.x));
         acc.y = __fma_rn(x.x, w.y, __fma_rn(x.y, w.x, acc.y));
       }
+      acc = c_add(a[t], acc);
       b[(t - j) * p + j + r * L] = acc;
     }
     next();

@@ -849,7 +849,6 @@ __global__ void __launch_bounds__(768) k_deposit_band(const double* __restrict__
 // longitudinal kick of dE besides.
 //
 // Bound by instruction issue, with the FP64 pipe (14 conversions and multiply-
-// Bound by instruction issue, with the FP64 pipe (14 conversions and multiply-
 // adds a particle, 28 with RB) close behind.  128 x 128 x 64: 1e6 particles in a
 // pipe 75 -> 48 us; 2e6 with RB, where a division and a logarithm held the FP64
 // pipe, 290 -> 112 us.  512, 640 and 768 threads are within 1%.
