@@ -127,16 +127,13 @@ MAP_FLOPS = {1: 22, 2: 16, 3: 25, 4: 70, 5: 70, 6: 18, 7: 25, 8: 20, 9: 14, 10: 
              14: 60, 15: 12, 16: 2, 17: 3, 18: 20, 19: 30, 20: 60}
 
 
-# FP64-pipe instructions per particle (thread level: DFMA, DMUL, DADD, the
-# conversions and compares) that the kernels execute on this workload,
-# counted by ncu (sm__inst_executed_pipe_fp64.sum x 32 / particles, 4e6
-# particles, the multiplies of the drift, quad fringe and bend maps on the
-# integer pipes): the fused pass alternates the {kick, quad1, quad2 (the
-# two back-to-back quad2 of the reference schedule merged), quad1,
-# fringe-out} segment (56.1) and the {kick, drift, fringe-in} segment
-# (38.1); the deposit runs 6.3 (one FMA per coordinate and the fixed-point
-# conversions; weights and sums are integer).
-FP64_INST_PER_PARTICLE = {"pass_kick_maps": (56.09 + 38.09) / 2, "deposit": 6.26}
+# FP64-pipe instructions per particle (thread level: multiply-adds and
+# conversions) that the kernels execute on this workload, counted by ncu
+# (sm__inst_executed_pipe_fp64 x 32 / particles, 4e6 particles): the
+# fixed-point pass runs 15 (the conversions of its coordinates), the deposit 6
+# (a multiply-add and a conversion per coordinate); the maps, weights and sums
+# are integer.
+FP64_INST_PER_PARTICLE = {"pass_kick_maps": 15.0, "deposit": 6.0}
 
 
 def pass_flops_per_turn(ops):
@@ -561,23 +558,22 @@ def run_ours(args):
                          "peak_source": "half the measured bf16 GEMM rate (MEASURED_PEAKS.json bf16_tflops)"
                          if bf16 else "half the fallback 1.9 PFLOP/s bf16"})
     if args.form in ("plain", "fp32") and name in ("pass_kick_maps", "pass_maps"):
-        # The fused pass keeps the maps in FP64 (both forms) and is bound by
-        # the FP64 pipe, not by HBM: its roof is the FP64 rate.  Algorithmic
-        # work = the reference's FP64 operation count of every map and SC
-        # kick the passes of one turn apply (FLOP-counting each +, -, *, /
-        # of teapotbase.cc and of the kick formulas), over the passes' time,
-        # against the DFMA rate measured in this process (2 FLOP per DFMA;
-        # MEASURED_PEAKS.json has no FP64 figure).  The deposit, gradient
-        # and extrema run on the integer pipes here, so the pass does the
-        # reference's work in fewer FP64 instructions than its count / 2
-        # and can read above 1.0.
+        # The fused pass is not bound by HBM: the FP32 form's maps run on the
+        # FP64 pipe, the plain form's in 64-bit fixed point on the integer
+        # pipes (bound by instruction issue).  Its algorithmic work is the
+        # reference's FP64 operation count of every map and SC kick the passes
+        # of one turn apply (FLOP-counting each +, -, *, / of teapotbase.cc and
+        # of the kick formulas), over the passes' time, against the DFMA rate
+        # measured in this process (2 FLOP per DFMA; MEASURED_PEAKS.json has no
+        # FP64 figure): what the same operations would take on the FP64 pipe,
+        # so the fixed-point pass reads above 1.0.
         hbm = dict(roofline)
         hbm.pop("kernels", None)
         pass_ms = sum(v[0] for k, v in prof.items() if k in ("pass_kick_maps", "pass_maps"))
         flops_turn = pass_flops_per_turn(prog.ops) * float(n)
         tflops = flops_turn / (pass_ms * 1e-3) / 1e12
         roofline.update({
-            "bound": "fp64", "kernel": "fused pass (kick + maps + extrema), all launches of one turn",
+            "bound": "issue" if args.form == "plain" else "fp64", "kernel": "fused pass (kick + maps + extrema), all launches of one turn",
             "achieved": tflops, "peak": fp64_peak, "unit": "TFLOP/s", "frac": tflops / fp64_peak,
             "peak_source": "measured in this run (orbit_device_peaks: independent DFMA chains on every SM, "
                            "2 FLOP per DFMA); MEASURED_PEAKS.json carries no FP64 figure",
