@@ -1051,7 +1051,8 @@ __device__ __forceinline__ void deposit_particles(const DepFast* sd, const DepSl
 // Which particles a band looks at, by the order of the high words of the
 // doubles alone (widened by 1/16 cell, so none of its own is missed): those
 // whose centre row may be its own, and for the first band also those that may
-// lie outside the transverse grid.
+// lie outside the transverse grid.  Centre rows are clamped to [1, nx - 2], so
+// the owner of row 1 takes all below it and the owner of row nx - 2 all above.
 struct BandKeys {
   int xlo, xhi, ylo, yhi, xout;
 };
@@ -1063,8 +1064,8 @@ __device__ __forceinline__ int hi_key(double v) {
 
 __device__ __forceinline__ void load_band_keys(BandKeys* k, const ScState* st, int nx, const BandAcc& a) {
   const double dx = 1.0 / st->inv_dx, dy = 1.0 / st->inv_dy;
-  k->xlo = a.first ? -0x7fffffff - 1 : hi_key(st->xmin + (a.r0 - 0.5625) * dx);
-  k->xhi = a.r1 >= nx ? 0x7fffffff : hi_key(st->xmin + (a.r1 - 0.4375) * dx);
+  k->xlo = a.r0 <= 1 ? -0x7fffffff - 1 : hi_key(st->xmin + (a.r0 - 0.5625) * dx);
+  k->xhi = a.r1 >= nx - 1 ? 0x7fffffff : hi_key(st->xmin + (a.r1 - 0.4375) * dx);
   k->ylo = a.first ? hi_key(st->ymin + 0.0625 * dy) : -0x7fffffff - 1;
   k->yhi = a.first ? hi_key(st->ymax - 0.0625 * dy) : 0x7fffffff;
   k->xout = a.first ? hi_key(st->xmax - 0.0625 * dx) : 0x7fffffff;
