@@ -1116,6 +1116,7 @@ static __device__ __forceinline__ void deposit_band_particles(const DepFast* sd,
       flush(32);
       have -= 32;
       if (lane < have) mine[lane] = mine[32 + lane];
+      __syncwarp();  // the slots above `have` are written next
     }
   }
   flush(have);
