@@ -221,6 +221,12 @@ int orbit_sc2p5drb_beam(orbit_sc2p5d_t* c, double* abx);
  * transform, PoissonSolverFFT2D.cc:103-172) since the calculator was
  * created.  Waits for the last stream the calculator ran on. */
 int orbit_sc2p5d_counters(orbit_sc2p5d_t* c, long long* kicks, long long* green_rebuilds);
+/* No counterpart in the reference (diagnostic).  Of the lattice passes after
+ * this calculator's kicks that have a fixed-point form: the passes that ran in
+ * it, and the particles that its FP64 routines took (the ones such a pass
+ * declined, and all of the passes whose constants did not fit).  Waits as
+ * orbit_sc2p5d_counters. */
+int orbit_sc2p5d_pass_counters(orbit_sc2p5d_t* c, long long* passes_fixed, long long* particles_fp64);
 /* Grid2D::calcGradient + Grid1D::getValue at n host points with the current
  * grids (Grid2D.cc:212-256, Grid1D.cc:191-211). */
 int orbit_sc2p5d_fields(orbit_sc2p5d_t* c, int n, const double* x, const double* y, const double* z,

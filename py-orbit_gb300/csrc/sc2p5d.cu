@@ -2211,6 +2211,17 @@ int orbit_sc2p5d_counters(orbit_sc2p5d_t* c, long long* kicks, long long* green_
   return ORBIT_OK;
 }
 
+int orbit_sc2p5d_pass_counters(orbit_sc2p5d_t* c, long long* passes_fixed, long long* particles_fp64) {
+  if (!c || !passes_fixed || !particles_fp64)
+    return set_error(ORBIT_ERR_ARG, "orbit_sc2p5d_pass_counters: bad argument");
+  if (c->used) ORBIT_CUDA(cudaEventSynchronize(c->done));
+  ScState h;
+  ORBIT_CUDA(cudaMemcpy(&h, c->d_st, sizeof(h), cudaMemcpyDeviceToHost));
+  *passes_fixed = (long long)h.n_fixed;
+  *particles_fp64 = (long long)h.n_fp64;
+  return ORBIT_OK;
+}
+
 int orbit_sc2p5d_get_sizes(const orbit_sc2p5d_t* c, int* nx, int* ny, int* nz, int* form) {
   if (!c) return set_error(ORBIT_ERR_ARG, "orbit_sc2p5d_get_sizes: null handle");
   if (nx) *nx = c->nx;

@@ -32,6 +32,8 @@ struct ScState {
   // longitudinal kick (SpaceChargeCalc2p5Drb.cc:124-136, 226-254)
   double rb_xc, rb_yc, rb_a2, rb_inv_a2, rb_lin, rb_lout;
   unsigned long long n_kicks, n_green;                    // kicks solved, Green spectra rebuilt
+  unsigned long long n_fixed, n_fp64;                     // lattice passes run in fixed point, and the particles of
+                                                          // those with such a form that the FP64 routines took
   // learned closure: fallen back to the plain deposit (sticky), the last
   // check's relative rms potential difference, checks and fall-backs
   int dn_fallback;
@@ -250,7 +252,7 @@ double sc_rb_long_factor(const orbit_sync_t& s, double length);
 
 // Per-particle SC kick and extrema helpers used inside fused passes.
 struct KickArgs {
-  const ScState* st;
+  ScState* st;
   const double* phi;      // plain form
   const double* lam;
   const float* phi_f;     // fp32 form

@@ -240,6 +240,12 @@ class DeviceSC2p5D:
         call("orbit_sc2p5d_counters", self.h, ctypes.byref(k), ctypes.byref(g))
         return k.value, g.value
 
+    def pass_counters(self):
+        """(lattice passes run in fixed point, particles their FP64 routines took) since creation."""
+        f, p = ctypes.c_longlong(), ctypes.c_longlong()
+        call("orbit_sc2p5d_pass_counters", self.h, ctypes.byref(f), ctypes.byref(p))
+        return f.value, p.value
+
     def fields(self, x, y, z):
         x, y, z = (np.ascontiguousarray(a, dtype=np.float64) for a in (x, y, z))
         n = x.shape[0]

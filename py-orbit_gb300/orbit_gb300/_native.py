@@ -86,6 +86,7 @@ _SIGS = {
     "orbit_sc2p5d_set_fused_conv": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]),
     "orbit_sc2p5d_set_conv_wait": (ctypes.c_int, [_vp, ctypes.c_longlong, ctypes.c_int]),
     "orbit_sc2p5d_counters": (ctypes.c_int, [_vp, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]),
+    "orbit_sc2p5d_pass_counters": (ctypes.c_int, [_vp, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]),
     "orbit_sc2p5drb_create": (ctypes.c_int, [ctypes.POINTER(_vp), ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                              ctypes.c_double]),
     "orbit_sc2p5drb_track": (ctypes.c_int, [_vp, _vp, ctypes.c_double, ctypes.c_double]),
