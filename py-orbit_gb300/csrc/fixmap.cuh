@@ -11,17 +11,21 @@
 // instructions (three 32 x 32 + 64-bit multiply-adds and a shift) and a sum
 // of products about three more per term, with one rounding at the end.
 //
-// Accuracy.  The scales put the bunch's bound at 2^61 units at most, so a
-// rounding is 2^-61 of the bound where binary64 rounds by 2^-53 of the value:
-// smaller for every particle within 2^-8 of the bound.  The bound is the
-// extent or 128 times the geometric mean of the magnitudes, whichever is less,
-// so a few far particles cannot coarsen the others' units; a particle beyond
-// it, one whose kick exceeds the momentum bound, and one with |dp_p| >= 1/8
-// take the FP64 routines, and so does the whole pass where the maps' constants
-// do not fit the scales (prep_pass).
-//
-// Measured rms error of x and xp over random segments: 7e-19 of the bound,
-// binary64's on the same particles 1.2e-16.
+// Accuracy.  The scales put the bunch's bound at 2^61 units at most: a rounding
+// is 2^-61 of the bound where binary64 rounds by 2^-53 of the value.  One scale
+// serves both planes and every particle, so it has to suit the smallest of x
+// and y (xp and yp) at its typical size, the geometric mean of the magnitudes
+// followed through the maps: the pass runs in fixed point only where each keeps
+// the 2^53 units of a double (fx::fine_enough).  Round beams have 2^55 to 2^58
+// of either, which is the room for planes apart.  Gaussian beams through random drifts, quadrupoles with fringes,
+// sextupoles and bends, planes up to a factor of 1e5 apart: the rms error of
+// each coordinate over binary64's on the same particles, by its typical size in
+// units: 2^55 0.45, 2^54 0.47 (at most 1.03), 2^53 0.57 (1.13), 2^52 0.68 (1.3),
+// 2^50 1.7 (3.6), 2^48 6.0.  The bound is the extent or 16 to 32 times the
+// geometric mean, whichever is less, so a few far particles cannot coarsen the
+// others' units; a particle beyond it, one whose kick exceeds a quarter of the
+// momentum bound, and one with |dp_p| >= 1/8 take the FP64 routines, and so does
+// the whole pass where the maps' constants do not fit the scales (prep_pass).
 //
 // The functions are __host__ __device__: a host build checks them against
 // extended-precision maps.
@@ -235,6 +239,12 @@ struct Bounds {
   int bad;
 };
 
+// Typical magnitudes of |x|, |xp|, |y|, |yp|, each by itself: the larger of a
+// map's terms, from below.
+struct Typical {
+  float x, p, y, r;
+};
+
 FX_HD float fmaxf_(float a, float b) { return a > b ? a : b; }
 
 // Whether the map has a fixed-point form.
@@ -275,6 +285,7 @@ inline void z_terms(const DevOp& o, double g2, double v[3]) {
 // g2 = 1/gamma^2.
 inline void compile_fixed(DevOp& o, double g2) {
   auto up = [](double a) { return (float)(std::fabs(a) * 1.0001); };
+  auto ups = [](double a) { return (float)(a * 1.0001); };
   const double* c = o.c;
   std::memset(o.f, 0, sizeof(o.f));
   std::memset(o.v, 0, sizeof(o.v));
@@ -287,10 +298,12 @@ inline void compile_fixed(DevOp& o, double g2) {
       v[1] = 0.5 * c[0];
       break;
     case ORBIT_OP_QUAD1:
-      f[0] = fmaxf_(up(c[0] - 1.0), up(c[4] - 1.0));
-      f[1] = fmaxf_(up(c[1]), up(c[5]));
-      f[2] = fmaxf_(up(c[2]), up(c[6]));
-      f[3] = fmaxf_(up(c[3] - 1.0), up(c[7] - 1.0));
+      for (int i = 0; i < 8; i += 4) {  // the planes
+        f[i] = ups(c[i] - 1.0);
+        f[i + 1] = up(c[i + 1]);
+        f[i + 2] = up(c[i + 2]);
+        f[i + 3] = ups(c[i + 3] - 1.0);
+      }
       for (int i = 0; i < 8; ++i) v[i] = c[i];
       v[0] -= 1.0;
       v[3] -= 1.0;
@@ -304,11 +317,11 @@ inline void compile_fixed(DevOp& o, double g2) {
       v[2] = 1.0;
       break;
     case ORBIT_OP_BEND1:
-      f[0] = up(c[0] - 1.0);
+      f[0] = ups(c[0] - 1.0);
       f[1] = up(c[1]);
       f[2] = up(c[2]);
       f[3] = up(c[3]);
-      f[4] = up(c[4] - 1.0);
+      f[4] = ups(c[4] - 1.0);
       f[5] = up(c[5]);
       f[6] = up(c[9]);
       for (int i = 0; i < 6; ++i) v[i] = c[i];
@@ -336,6 +349,7 @@ inline void compile_fixed(DevOp& o, double g2) {
       break;
     case ORBIT_OP_MULTP:
       f[0] = up(c[0]);
+      f[1] = o.i1 ? 1.f : 0.f;
       v[0] = c[0];
       break;
     case ORBIT_OP_MPFRIN: case ORBIT_OP_MPFROUT:
@@ -346,7 +360,8 @@ inline void compile_fixed(DevOp& o, double g2) {
       o.i2 = c[0] != 0.0 ? 0 : 1;
       break;
     case ORBIT_OP_KICK:
-      f[0] = fmaxf_(up(c[0]), up(c[1]));
+      f[0] = up(c[0]);
+      f[1] = up(c[1]);
       v[0] = c[0];
       v[1] = c[1];
       break;
@@ -385,12 +400,14 @@ FX_HD void bound_op(int code, int i0, const float* f, Bounds& b) {
       b.x = x + kb * f[0] * p;
       b.xp = fmaxf_(b.xp, f[0]);
       break;
-    case ORBIT_OP_QUAD1:
-      b.x = x * (1.0f + f[0]) + f[1] * p;
-      b.p = p * (1.0f + f[3]) + f[2] * x;
-      b.xp = fmaxf_(b.xp, f[1]);
-      b.px = fmaxf_(b.px, f[2]);
+    case ORBIT_OP_QUAD1: {
+      const float xp = fmaxf_(f[1], f[5]), px = fmaxf_(f[2], f[6]);
+      b.x = x * (1.0f + fmaxf_(fabsf(f[0]), fabsf(f[4]))) + xp * p;
+      b.p = p * (1.0f + fmaxf_(fabsf(f[3]), fabsf(f[7]))) + px * x;
+      b.xp = fmaxf_(b.xp, xp);
+      b.px = fmaxf_(b.px, px);
       break;
+    }
     case ORBIT_OP_QUAD2:
     case ORBIT_OP_BEND2:
       b.x = x + kb * b.dp * f[0] * p;
@@ -403,8 +420,8 @@ FX_HD void bound_op(int code, int i0, const float* f, Bounds& b) {
       b.p = p * 1.02f;
       break;
     case ORBIT_OP_BEND1:
-      b.x = fmaxf_(x * (1.0f + f[0]) + f[1] * p + f[2] * b.dp, x + f[6] * p);
-      b.p = p * (1.0f + f[4]) + f[3] * x + f[5] * b.dp;
+      b.x = fmaxf_(x * (1.0f + fabsf(f[0])) + f[1] * p + f[2] * b.dp, x + f[6] * p);
+      b.p = p * (1.0f + fabsf(f[4])) + f[3] * x + f[5] * b.dp;
       b.xp = fmaxf_(b.xp, fmaxf_(f[1], f[6]));
       b.px = fmaxf_(b.px, f[3]);
       break;
@@ -439,7 +456,44 @@ FX_HD void bound_op(int code, int i0, const float* f, Bounds& b) {
       break;
     }
     case ORBIT_OP_KICK:
-      b.p = p + f[0];
+      b.p = p + fmaxf_(f[0], f[1]);
+      break;
+    default:
+      break;
+  }
+}
+
+// The same for the typical magnitudes.
+FX_HD void typical_op(int code, int i0, const float* f, Typical& t) {
+  const Typical o = t;
+  switch (code) {
+    case ORBIT_OP_DRIFT:
+      t.x = fmaxf_(o.x, f[0] * o.p);
+      t.y = fmaxf_(o.y, f[0] * o.r);
+      break;
+    case ORBIT_OP_QUAD1:
+      t.x = fmaxf_(o.x * fabsf(1.0f + f[0]), f[1] * o.p);
+      t.p = fmaxf_(o.p * fabsf(1.0f + f[3]), f[2] * o.x);
+      t.y = fmaxf_(o.y * fabsf(1.0f + f[4]), f[5] * o.r);
+      t.r = fmaxf_(o.r * fabsf(1.0f + f[7]), f[6] * o.y);
+      break;
+    case ORBIT_OP_BEND1:
+      t.x = fmaxf_(o.x * fabsf(1.0f + f[0]), f[1] * o.p);
+      t.p = fmaxf_(o.p * fabsf(1.0f + f[4]), f[3] * o.x);
+      t.y = fmaxf_(o.y, f[6] * o.r);
+      break;
+    case ORBIT_OP_MULTP: {
+      float a = 1.0f, b = 0.0f;  // |z^n|'s parts
+      if (i0 == 1) a = o.x, b = o.y;
+      if (i0 == 2) a = fmaxf_(o.x * o.x, o.y * o.y), b = 2.0f * o.x * o.y;
+      if (i0 == 3) a = o.x * fmaxf_(o.x * o.x, 3.0f * o.y * o.y), b = o.y * fmaxf_(o.y * o.y, 3.0f * o.x * o.x);
+      t.p = fmaxf_(o.p, f[0] * (f[1] != 0.0f ? b : a));
+      t.r = fmaxf_(o.r, f[0] * (f[1] != 0.0f ? a : b));
+      break;
+    }
+    case ORBIT_OP_KICK:
+      t.p = fmaxf_(o.p, f[0]);
+      t.r = fmaxf_(o.r, f[1]);
       break;
     default:
       break;
@@ -477,15 +531,25 @@ FX_HD bool fixk(double v, int F, V* out, int* k) {
   return ok;
 }
 
-// Sx, Sp and k from the bounds after the last map: the finest units; false
-// when the maps mix x and p too strongly for them.
+// Sx, Sp and k from the bounds after the last map: the finest units, or coarser
+// ones of the coordinate whose coefficients would not fit beside the other's;
+// false when the maps mix x and p too strongly for any.
 FX_HD bool choose_scales(const Bounds& b, Scales& s) {
   if (b.bad || !(b.x > 0.0f) || !(b.p > 0.0f) || !(b.x < 1e6f) || !(b.p < 1e3f) || !(b.dp < 0.15f)) return false;
   s.x = 61 - exp_above(b.x);
   s.p = 61 - exp_above(b.p);
+  const int xp = exp_above(b.xp), px = exp_above(b.px);
+  if (px + s.p - s.x > 3) s.p = 3 + s.x - px;
+  if (xp + s.x - s.p > 3) s.x = 3 + s.p - xp;
   const int k = 61 - exp_above(b.dp * 1.2f);
   s.k = k < 64 ? 64 : (k > 80 ? 80 : k);
-  return s.x <= 100 && s.p <= 100 && exp_above(b.xp) + s.x - s.p <= 3 && exp_above(b.px) + s.p - s.x <= 3;
+  return s.x <= 100 && s.p <= 100 && xp + s.x - s.p <= 3 && px + s.p - s.x <= 3;
+}
+
+// The scales suit the typical magnitudes after the last map.
+FX_HD bool fine_enough(const Typical& t, const Scales& s) {
+  const float x = t.x < t.y ? t.x : t.y, p = t.p < t.r ? t.p : t.r;
+  return exp_above(x) + s.x > 53 && exp_above(p) + s.p > 53;
 }
 
 // Left shift of z^n before the multipole kick's product.

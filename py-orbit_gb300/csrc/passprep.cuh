@@ -45,40 +45,59 @@ static __device__ __noinline__ void prep_pass(const PrepJob& J, const ScState* s
   const int lane = threadIdx.x & 31, nops = J.b - J.a;
   FxPass* f = &J.out->fx;
   // lane 0 the segment's start entry, lanes 1..nops its maps
-  bool ok = nops < fx::kMaxOps && st->mag.pmax != 0u && st->mag.n != 0u && !st->skip;
+  bool ok = nops < fx::kMaxOps && st->mag.pmax != 0u && !st->skip;
   const DevOp* o = J.ops + J.a - 1 + (lane <= nops ? lane : 0);
   const int code = lane <= nops ? o->code : 0, i0 = lane <= nops ? o->i0 : 0;
-  float c[7];
+  float c[8];
 #pragma unroll
-  for (int q = 0; q < 7; ++q) c[q] = lane <= nops ? o->f[q] : 0.f;
-  // bounds: the extent, or 128 times the geometric mean of the magnitudes
+  for (int q = 0; q < 8; ++q) c[q] = lane <= nops ? o->f[q] : 0.f;
+  // typical magnitudes of x, xp, y, yp: the geometric mean of those that are not
+  // zero, which have to be half of the sample
+  unsigned cnt[4], most = 1u;
+  float mean[4];
+  for (int q = 0; q < 4; ++q) {
+    cnt[q] = (unsigned)(st->mag.exp[q] >> 32);
+    mean[q] = (float)(unsigned)st->mag.exp[q] / (float)max(cnt[q], 1u) - 60.f;
+    most = max(most, cnt[q]);
+  }
+  for (int q = 0; q < 4; ++q) ok = ok && 2u * cnt[q] >= most;
+  fx::Typical ty = {exp2f(mean[0]), exp2f(mean[1]), exp2f(mean[2]), exp2f(mean[3])};
+  // bounds: the extent, or 16 to 32 times the larger plane's typical magnitude
   // where a few particles lie further out
-  const float inv = 0.5f / (float)st->mag.n;
-  const int ex = (int)floorf((float)st->mag.sx * inv) - 1023 + 8, ep = (int)floorf((float)st->mag.sp * inv) - 1023 + 8;
+  const int ex = (int)floorf(fmaxf(mean[0], mean[2])) + 5, ep = (int)floorf(fmaxf(mean[1], mean[3])) + 5;
   const float xm = (float)st->mag.xmax * 1.0001f;
   const float pm = (float)__hiloint2double((int)st->mag.pmax, -1) * 1.0001f;
   const float dm = (float)__hiloint2double((int)st->mag.emax, -1) * fabsf((float)J.dp_p_coeff) * 1.0001f;
   const float x0 = fminf(xm, ldexpf(1.f, ex)), p0 = fminf(pm, ldexpf(1.f, ep)), d0 = fminf(dm, 0.124f);
-  fx::Bounds bd = {x0, 2.f * p0, d0, 0.f, 0.f, 0};
+  fx::Bounds bd = {x0, 1.25f * p0, d0, 0.f, 0.f, 0};
   if (ok) {
     for (int q = 1; q <= nops; ++q) {
-      float g[7];
+      float g[8];
 #pragma unroll
-      for (int w = 0; w < 7; ++w) g[w] = __shfl_sync(0xffffffffu, c[w], q);
-      fx::bound_op(__shfl_sync(0xffffffffu, code, q), __shfl_sync(0xffffffffu, i0, q), g, bd);
+      for (int w = 0; w < 8; ++w) g[w] = __shfl_sync(0xffffffffu, c[w], q);
+      const int cq = __shfl_sync(0xffffffffu, code, q), iq = __shfl_sync(0xffffffffu, i0, q);
+      fx::bound_op(cq, iq, g, bd);
+      fx::typical_op(cq, iq, g, ty);
     }
     fx::Scales s;
     ok = fx::choose_scales(bd, s);
-    fx::Op out;
-    out.bad = 0;
-    int md = 80;
-    if (ok && lane <= nops) md = fx::consts_op(*o, s, out, true);
-    s.d = __reduce_min_sync(0xffffffffu, md);
-    if (ok && lane <= nops) {
-      fx::consts_op(*o, s, out, false);
-      f->op[lane] = out;
+    // a constant too large for the units of xp (a sextupole's, for a beam with
+    // little slope) may fit coarser ones
+    for (int t = 0; ok; ++t, --s.p) {
+      ok = fx::fine_enough(ty, s);
+      fx::Op out;
+      out.bad = 0;
+      int md = 80;
+      if (ok && lane <= nops) md = fx::consts_op(*o, s, out, true);
+      s.d = __reduce_min_sync(0xffffffffu, md);
+      if (ok && lane <= nops) {
+        fx::consts_op(*o, s, out, false);
+        f->op[lane] = out;
+      }
+      const bool fits = __all_sync(0xffffffffu, ok && out.bad == 0 && s.d >= 50);
+      if (fits) break;
+      ok = ok && t < 2;
     }
-    ok = __all_sync(0xffffffffu, ok && out.bad == 0 && s.d >= 50);
     if (lane == 0 && ok) {
       f->n = nops;
       f->s = s;
@@ -86,21 +105,22 @@ static __device__ __noinline__ void prep_pass(const PrepJob& J, const ScState* s
       f->limx = __double2hiint((double)x0);
       f->limp = __double2hiint((double)p0);
       f->limd = __double2hiint((double)d0);
-      int64_t v;  // a kick of at most the momentum bound
-      if (!fx::fixc((double)p0, s.p, &v)) ok = false;
+      int64_t v;  // a kick of at most a quarter of the momentum bound
+      if (!fx::fixc(0.25 * (double)p0, s.p, &v)) ok = false;
       f->limk = (int)(v >> 32);
       auto width = [](int ncell) {
         int w = 0;
         while ((1 << w) < ncell + 2) ++w;
         return w;
       };
-      // grid coordinate in units of 2^-F, at most 2^57
+      // grid coordinate in units of 2^-F, at most 2^57; no coarser than binary64
+      // at the far edge
       auto grid = [&](double inv_d, double cc, int ncell, FxGrid* g) {
         int ff = 57 - width(ncell);
         const int room = 61 - fx::exp_of(inv_d) + s.x - 64;
         if (room < ff) ff = room;
         int64_t t;
-        if (ff < 40 || !fx::fixv(inv_d, ff - s.x + 64, &g->a) || !fx::fixc(cc - 0.5, ff, &t)) {
+        if (ff < 53 - width(ncell) || !fx::fixv(inv_d, ff - s.x + 64, &g->a) || !fx::fixc(cc - 0.5, ff, &t)) {
           ok = false;
           return;
         }

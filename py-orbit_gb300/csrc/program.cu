@@ -106,7 +106,7 @@ struct FxFallback {
   const DevOp* ops;
   int a, b;
   unsigned long long mn[3], mx[3];
-  unsigned pm, sx, sp, n;
+  unsigned pm, ex[4];  // (ex: MagAcc::part sums)
   int bad;
   unsigned taken;  // particles the FP64 routines took
 };
@@ -138,12 +138,11 @@ __device__ __noinline__ void pass_particle(FxFallback* f, int i, bool first) {
     if (e.bad) f->bad = 1;
     MagAcc g;
     g.init();
-    g.add(p.x, p.xp, p.y, p.yp, p.dE);
+    g.bound(p.xp, p.yp);
     atomicMax(&f->pm, g.pm);
     if (first) {
-      atomicAdd(&f->sx, g.sx);
-      atomicAdd(&f->sp, g.sp);
-      atomicAdd(&f->n, g.n);
+      g.sample(p.x, p.xp, p.y, p.yp);
+      for (int c = 0; c < 4; ++c) atomicAdd(&f->ex[c], g.part(c));
     }
   }
   f->c[0][i] = p.x; f->c[1][i] = p.xp; f->c[2][i] = p.y; f->c[3][i] = p.yp; f->c[4][i] = p.z;
@@ -327,7 +326,7 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
       s_f.k = &s_prep.k; s_f.kf = &s_prep.kf;
       s_f.dE = cdE; s_f.knl = knl_buf; s_f.kick = &kick; s_f.m = &m; s_f.ops = ops; s_f.a = a; s_f.b = b;
       for (int c = 0; c < 3; ++c) { s_f.mn[c] = ~0ull; s_f.mx[c] = 0ull; }
-      s_f.pm = s_f.sx = s_f.sp = s_f.n = 0u;
+      s_f.pm = s_f.ex[0] = s_f.ex[1] = s_f.ex[2] = s_f.ex[3] = 0u;
       s_f.bad = 0;
       s_f.taken = 0u;
     }
@@ -415,11 +414,8 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
       mag.pm = max(mag.pm, s_f.pm);
       // dE is unchanged; without magnitudes before, none are claimed
       mag.em = kick.st->mag.pmax ? kick.st->mag.emax : 0x7fefffffu;
-      mag.sx += s_f.sx;
-      mag.sp += s_f.sp;
-      mag.n += s_f.n;
     }
-    if (sa.mag) mag_block_commit(mag, ext_st);
+    if (sa.mag) mag_block_commit(mag, ext_st, s_f.ex);
     ext_commit_and_setup(acc, ext_st, status, sa, nblk);
   }
 }

@@ -44,14 +44,15 @@ struct ScState {
   unsigned conv_bar[2];
   // magnitudes of the bunch for the fixed-point maps of the next pass,
   // accumulated by a lattice pass beside the extrema: largest high words of
-  // |xp|, |yp| and of |dE|, sums of the clamped exponents of x, y and of xp,
-  // yp over every thread's first particle and their number; the set-up moves
-  // them to `mag` (zero after a scan that has none)
-  unsigned acc_pmax, acc_emax, acc_n;
-  unsigned long long acc_sx, acc_sp;
+  // |xp|, |yp| and of |dE|; of x, xp, y, yp the sums of the exponents (clamped
+  // to 2^-60..2^60, from 0) over one particle of every thread, with the number
+  // of those that are not zero above them (2^32); the set-up moves them to `mag`
+  // (zero after a scan that has none)
+  unsigned acc_pmax, acc_emax;
+  unsigned long long acc_exp[4];
   struct {
-    unsigned pmax, emax, n;
-    unsigned long long sx, sp;
+    unsigned pmax, emax;
+    unsigned long long exp[4];
     double xmax;  // max |x|, |y| before the grid is stretched
   } mag;
 };
