@@ -481,6 +481,7 @@ __device__ __forceinline__ void kick_plain(const KickConst& k, const double* __r
   yp += gy * k.inv_dy * lf;
 }
 
+// FP32 form: gradient and line density in FP32, accumulation into FP64.
 __device__ __forceinline__ void kick_fp32(const KickConst& k, const float* __restrict__ phi,
                                           const float* __restrict__ lam, double x, double y, double z,
                                           double& xp, double& yp) {
@@ -1153,25 +1154,6 @@ __device__ __forceinline__ void load_kick_fix(KickFix& k, const ScState* st, dou
   k.nx = nx; k.ny = ny; k.nz = nz;
   k.Fx = fix_bits(nx); k.Fy = fix_bits(ny); k.Fz = fix_bits(nz);
   k.skip = st->skip;
-}
-
-// The kick constants computed once per block (thread 0) and copied to every
-// thread: a thread of a 512-thread block handles only ~13 particles of a
-// 1e6-particle bunch, and the set-up holds two FP64 divisions, which on
-// GB300 occupy the FP64 pipe that bounds the fused pass.  (Reading the
-// constants from shared memory inside the particle loop instead spills
-// registers there and is slower.)  Every thread of the block must call it.
-__device__ __forceinline__ void load_kick_block(KickConst& k, KickFix* kf, const ScState* st, double host_factor,
-                                                int nx, int ny, int nz) {
-  __shared__ KickConst s_k;
-  __shared__ KickFix s_kf;
-  if (threadIdx.x == 0) {
-    load_kick_const(s_k, st, host_factor, nx, ny, nz);
-    if (kf) load_kick_fix(s_kf, st, s_k.fac, nx, ny, nz);
-  }
-  __syncthreads();
-  k = s_k;
-  if (kf) *kf = s_kf;
 }
 
 __device__ __forceinline__ long long phi_fixed(double v, int s) {
