@@ -39,6 +39,9 @@ enum : unsigned {
 
 int num_sms();
 
+// Shared memory of one block, static and dynamic together.
+static const size_t kBlockSmem = 227 * 1024;
+
 // Optional per-launch timing (orbit_program_profile): when a profiler is
 // installed on the calling thread, every launch site brackets its kernel
 // with a pair of CUDA events on the launching stream.

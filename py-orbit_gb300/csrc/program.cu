@@ -111,6 +111,9 @@ struct FxFallback {
   unsigned taken;  // particles the FP64 routines took
 };
 
+static_assert(kPassSmem + sizeof(FxFallback) + sizeof(PassPrep) + kCommitSmem + 64 <= kBlockSmem,
+              "k_pass_fx: its own shared memory beside the largest copy of the potential");
+
 // One particle by the FP64 routines: those the fixed-point form declines,
 // and all of a pass it cannot run.
 template <bool EXT>

@@ -844,6 +844,12 @@ __global__ void __launch_bounds__(768) k_deposit_band(const double* __restrict__
                     blockIdx.x / nb, gridDim.x / nb);
 }
 
+static_assert(kMaxSmem + sizeof(DepFast) + sizeof(DepSlow<BandAcc, GridAcc<true>>) + sizeof(BandKeys) +
+                      64 * (768 / 32) * sizeof(int) + 64 <= kBlockSmem,
+              "k_deposit_band: its own shared memory beside the largest band");
+static_assert(kMaxSmem + sizeof(KickConst) + sizeof(KickFix) + sizeof(KickDirect) + sizeof(LogTab) + 64 <= kBlockSmem,
+              "k_kick_plain: its own shared memory beside the largest copy of the potential");
+
 // Kick (SpaceChargeCalc2p5D.cc:104-119): fixed-point gradient and line
 // density (kick_direct), FP64 routine for the particles it declines.  RB: the
 // longitudinal kick of dE besides.

@@ -88,6 +88,9 @@ __device__ __forceinline__ void mag_block_commit(const MagAcc& a, ScState* st, c
   }
 }
 
+// Static shared memory of mag_block_commit, ext_block_commit and last_block_done.
+static const size_t kCommitSmem = 6 * 32 * (sizeof(unsigned) + sizeof(unsigned long long)) + 16;
+
 // Smallest 64-bit key of a warp, from two 32-bit reductions.
 __device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
   const unsigned h = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32));
