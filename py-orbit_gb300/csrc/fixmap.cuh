@@ -178,7 +178,28 @@ FX_HD bool fixv(double v, int F, V* out) {
   return ok;
 }
 
-// x 2^S truncated, for |x| 2^S < 2^62 (false otherwise).
+// x 2^S to the nearest integer and back, by the conversion instructions (the
+// power of two joins the exponent): the FP64 pipe is otherwise idle in the
+// fixed-point pass.
+FX_HD int64_t cvt_to(double x, int S) {
+#ifdef __CUDA_ARCH__
+  return __double2ll_rn(__hiloint2double(__double2hiint(x) + (S << 20), __double2loint(x)));
+#else
+  return (int64_t)std::llrint(sf::from_bits(sf::bits(x) + ((uint64_t)(int64_t)S << 52)));
+#endif
+}
+FX_HD double cvt_from(int64_t v, int S) {
+#ifdef __CUDA_ARCH__
+  const double d = __ll2double_rn(v);
+  const int h = __double2hiint(d);
+  return __hiloint2double(h == 0 ? 0 : h - (S << 20), __double2loint(d));
+#else
+  const uint64_t u = sf::bits((double)v);
+  return sf::from_bits(u == 0 ? 0 : u - ((uint64_t)(int64_t)S << 52));
+#endif
+}
+
+// x 2^S truncated, for |x| 2^S < 2^62 (false otherwise); of the host check.
 FX_HD bool to_fix(double x, int S, int64_t* out) {
   const uint64_t u = sf::bits(x);
   int r = 1085 - S - ((int)(u >> 52) & 0x7FF);

@@ -41,18 +41,6 @@ __device__ __noinline__ void kick_consts_into(KickConst* k, KickFix* kf, const K
   if (kf) load_kick_fix(*kf, kick.st, k->fac, kick.nx, kick.ny, kick.nz);
 }
 
-// x 2^S to the nearest integer and back, by the conversion instructions (the
-// power of two joins the exponent): the FP64 pipe is otherwise idle in the
-// fixed-point pass.
-__device__ __forceinline__ long long cvt_to(double x, int S) {
-  return __double2ll_rn(__hiloint2double(__double2hiint(x) + (S << 20), __double2loint(x)));
-}
-__device__ __forceinline__ double cvt_from(long long v, int S) {
-  const double d = __ll2double_rn(v);
-  const int h = __double2hiint(d);
-  return __hiloint2double(h == 0 ? 0 : h - (S << 20), __double2loint(d));
-}
-
 // Cell and fraction (Q62) of tsc_fixed; false within a quarter cell of the
 // grid's edge or outside.
 __device__ __forceinline__ bool cell_fx(const FxGrid& g, long long x, int ncell, int& ic, long long& f) {
@@ -73,7 +61,7 @@ __device__ __forceinline__ bool kick_fx(const FxPass& f, int nx, const long long
   const bool in = cell_fx(f.gx, t.x, nx, ix, gfx) & cell_fx(f.gy, t.y, f.ny, iy, gfy);
   if (!in) return false;
   if (f.nz > 1) {
-    const long long v = cvt_to(fma(t.z, f.az, f.cz), f.Fz);
+    const long long v = fx::cvt_to(fma(t.z, f.az, f.cz), f.Fz);
     const int i = min(max((int)(v >> f.Fz), 0), f.nz);
     const long long w = (long long)((unsigned long long)(v - ((long long)i << f.Fz)) << (62 - f.Fz));
     lv = fx::mul2(fx::sp((1ll << 62) - w), fx_of_pair(Lm[(i == 0 ? f.nz : i) - 1]), fx::sp(w),
@@ -175,8 +163,8 @@ struct ExtFx {
   __device__ __forceinline__ void join(ExtAcc& a, int S) const {
     for (int c = 0; c < 2; ++c) {
       if (mn[c] > mx[c]) continue;
-      a.mn[c] = dkey(cvt_from(mn[c], S));
-      a.mx[c] = dkey(cvt_from(mx[c], S));
+      a.mn[c] = dkey(fx::cvt_from(mn[c], S));
+      a.mx[c] = dkey(fx::cvt_from(mx[c], S));
     }
     a.mn[2] = zn;
     a.mx[2] = zx;
@@ -362,10 +350,10 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
       const double knl = knl_buf[i];  // as an earlier pass of this run computed it from the same dE
       const double dp = __dmul_rn(dE, m.dp_p_coeff);
       t.z = cz[i];
-      t.x = cvt_to(x0, s.x);
-      t.p = cvt_to(xp0, s.p);
-      t.y = cvt_to(y0, s.x);
-      t.r = cvt_to(yp0, s.p);
+      t.x = fx::cvt_to(x0, s.x);
+      t.p = fx::cvt_to(xp0, s.p);
+      t.y = fx::cvt_to(y0, s.x);
+      t.r = fx::cvt_to(yp0, s.p);
       bool ok = true;
       if (s_fx.check) {
         auto inside = [](double v, int lim) { return (__double2hiint(v) & 0x7fffffff) <= lim; };
@@ -380,10 +368,10 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
         ++todo;
         continue;
       }
-      fx::part_init(t, fx::kappa_of(knl), cvt_to(dp, s.k), s.k);
+      fx::part_init(t, fx::kappa_of(knl), fx::cvt_to(dp, s.k), s.k);
       fx::apply(t, s_fx.op, s_fx.n, s);
-      const double x = cvt_from(t.x, s.x), xp = cvt_from(t.p, s.p), y = cvt_from(t.y, s.x), yp = cvt_from(t.r, s.p);
-      const double z = t.z + cvt_from(t.d, s.d);
+      const double x = fx::cvt_from(t.x, s.x), xp = fx::cvt_from(t.p, s.p), y = fx::cvt_from(t.y, s.x), yp = fx::cvt_from(t.r, s.p);
+      const double z = t.z + fx::cvt_from(t.d, s.d);
       if (EXT) {
         ext.add(t.x, t.y, z);
         mag.bound(xp, yp);

@@ -102,7 +102,16 @@ int main(int argc, char** argv) {
     for (auto& B : beam) {
       const double knl = 1.0 / (1.0 + B.dp);
       const L dp = 1.0L / (L)knl - 1.0L;
-      auto fix = [](double v, int S) { return (int64_t)std::llrint(std::ldexp((L)v, S)); };
+      auto fix = [](double v, int S) {  // the kernel's conversions: half a unit in, half an ulp back
+        const int64_t f = fx::cvt_to(v, S);
+        const double o = fx::cvt_from(f, S);
+        if (std::fabs((L)f - std::ldexp((L)v, S)) > 0.5L ||
+            std::fabs((L)o - std::ldexp((L)f, -S)) > std::fabs((L)o) * std::ldexp(1.0L, -53) * 1.0000001L) {
+          std::printf("conversion off\n");
+          std::exit(1);
+        }
+        return f;
+      };
       fx::Part f;
       f.x = fix(B.x, sc.x); f.p = fix(B.p, sc.p); f.y = fix(B.y, sc.x); f.r = fix(B.r, sc.p); f.z = B.z;
       fx::part_init(f, fx::kappa_of(knl), fix((double)dp, sc.k), sc.k);
@@ -110,7 +119,7 @@ int main(int argc, char** argv) {
       P<double> D = {B.x, B.p, B.y, B.r, B.z, (double)dp};
       for (int k = 1; k <= n; ++k) { map<L>(T, seg[k], g2); map<double>(D, seg[k], g2); }
       fx::apply(f, fo.data(), n, sc);
-      const double o[4] = {fx::from_fix(f.x, sc.x), fx::from_fix(f.p, sc.p), fx::from_fix(f.y, sc.x), fx::from_fix(f.r, sc.p)};
+      const double o[4] = {fx::cvt_from(f.x, sc.x), fx::cvt_from(f.p, sc.p), fx::cvt_from(f.y, sc.x), fx::cvt_from(f.r, sc.p)};
       const double d[4] = {D.x, D.p, D.y, D.r};
       const L w[4] = {T.x, T.p, T.y, T.r};
       for (int k = 0; k < 4; ++k) {
