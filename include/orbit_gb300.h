@@ -368,11 +368,13 @@ int orbit_batch_stream(orbit_batch_t* b, void** stream);
 int orbit_batch_profile(orbit_batch_t* b, int max_kinds, char* names, double* total_ms, int* launches,
                         int* nkinds);
 /* Class cls: grid[3] = nx, ny, nz; members; tuning[6] = deposit threads,
- * deposit particles per block, pass threads, pass particles per block, FFT
+ * deposit particles per block, pass threads (of a pass's FP64 form; the
+ * fixed-point form has a block size of its own), pass particles per block, FFT
  * schedule (1: radix-2 stages, 0: radix-4 stages), tuned (0/1). */
 int orbit_batch_class(const orbit_batch_t* b, int cls, int* grid, int* members, int* tuning);
-/* Fixes class cls's shapes (tuning[0..4], one of the candidates); no
- * autotuning runs afterwards. */
+/* Fixes class cls's shapes (tuning[0..4], one of the candidates or a shape
+ * that orbit_batch_class of any batch reported); no autotuning runs
+ * afterwards. */
 int orbit_batch_set_tuning(orbit_batch_t* b, int cls, const int* tuning);
 
 /* ---- NVTX ranges (no counterpart in the reference) ----

@@ -44,6 +44,7 @@ static const int kNPass = 4;
 // make one wave (one block per SM), or two.  A block's prologue (its copy of
 // the potential, the constants) is then paid once or twice per SM.
 static const int kNWave = 2;
+static const int kMinWaveChunk = 256;
 static const int kMaxDep = kNDep + kNWave, kMaxPass = kNPass + kNWave;
 
 struct BatchClass {
@@ -60,6 +61,7 @@ struct BatchClass {
   std::vector<BlockMap> pass_maps; // one per pass candidate
   int dep_cand[kMaxDep][2] = {}, pass_cand[kMaxPass][2] = {};  // {threads, particles per block}
   int dep_sel = 0, pass_sel = 0;
+  int dep_own = 0, pass_own = 0;   // particles per block set by hand, in place of the first wave shape
   std::string dep_tag, pass_tag;   // profile names of the class's deposit and kick passes
   cudaStream_t st = nullptr;
   cudaEvent_t joined = nullptr;
@@ -154,7 +156,7 @@ static int wave_chunk(const orbit_batch_t* bt, const BatchClass& c, int waves, i
     for (int m : c.mem) nb += std::max(1, (bt->bunches[m]->n + chunk - 1) / chunk);
     return nb;
   };
-  int lo = (int)std::max(256ll, total / std::max(1, cap)), hi = nmax;
+  int lo = (int)std::max((long long)kMinWaveChunk, total / std::max(1, cap)), hi = nmax;
   if (lo >= hi || blocks(hi) > cap) return std::max(lo, hi);
   while (lo < hi) {
     const int mid = lo + (hi - lo) / 2;
@@ -170,10 +172,12 @@ static void fill_candidates(const orbit_batch_t* bt, BatchClass& c) {
   for (int q = 0; q < kMaxDep; ++q) {
     c.dep_cand[q][0] = kDepCand[q < kNDep ? q : 0][0];
     c.dep_cand[q][1] = q < kNDep ? kDepCand[q][1] : wave_chunk(bt, c, 1 + q - kNDep, bands);
+    if (q == kNDep && c.dep_own > 0) c.dep_cand[q][1] = c.dep_own;
   }
   for (int q = 0; q < kMaxPass; ++q) {
     c.pass_cand[q][0] = ORBIT_PASS_THREADS;
     c.pass_cand[q][1] = q < kNPass ? kPassCand[q][1] : wave_chunk(bt, c, 1 + q - kNPass, 1);
+    if (q == kNPass && c.pass_own > 0) c.pass_cand[q][1] = c.pass_own;
   }
 }
 
@@ -191,7 +195,7 @@ static int build_map(const orbit_batch_t* bt, const BatchClass& c, int chunk, in
   std::vector<int2> mb(c.mem.size());
   for (size_t j = 0; j < c.mem.size(); ++j) {
     int n = bt->bunches[c.mem[j]]->n;
-    int nb = (n + chunk - 1) / chunk;
+    int nb = (int)(((long long)n + chunk - 1) / chunk);
     if (nb < 1) nb = 1;
     nb *= per;
     mb[j].x = (int)bj.size();
@@ -390,6 +394,8 @@ static int enqueue_class_turn(orbit_batch_t* bt, int ci, cudaStream_t s, bool pr
   auto pass = [&](int table, const Seg& sg, bool kick, bool ext, int cand, int km) -> int {
     Tuner* t = kick ? tu : nullptr;
     Tuner::Rec r{};
+    // relative work: a kick costs about as much as six maps (777 instructions a
+    // particle with one map, about 1300 with five)
     int rc = rec_begin(t, ci, 1, cand, (float)(6 + sg.b - sg.a), s, &r);
     if (rc) return rc;
     rc = batch_enqueue_pass(c.d_pass + (size_t)table * nm, c.pass_maps[cand], c.pass_cand[cand][0], kick ? 1 : 0, ext,
@@ -792,16 +798,25 @@ int orbit_batch_set_tuning(orbit_batch_t* bt, int cls, const int* tuning) {
   if (!bt || !tuning || cls < 0 || cls >= (int)bt->classes.size())
     return set_error(ORBIT_ERR_ARG, "orbit_batch_set_tuning: bad argument");
   BatchClass& c = bt->classes[cls];
-  int ds = -1, ps = -1;
-  if (!bt->compiled) fill_candidates(bt, c);  // a shape reported by another batch of the same bunches
-  auto is = [](const int cand[2], int threads, int chunk) { return cand[0] == threads && cand[1] == chunk; };
-  for (int q = kMaxDep - 1; q >= 0; --q)
-    if (is(c.dep_cand[q], tuning[0], tuning[1])) ds = q;
-  for (int q = kMaxPass - 1; q >= 0; --q)
-    if (is(c.pass_cand[q], tuning[2], tuning[3])) ps = q;
+  // one of the fixed shapes, or a wave shape that any batch has reported: those
+  // follow the bunches' sizes, so every number of particles per block that they
+  // can have is taken, and stays as it is when the sizes change
+  auto match = [](const int cand[][2], int n, const int* t, int* own) {
+    *own = 0;
+    for (int q = 0; q < n; ++q)
+      if (cand[q][0] == t[0] && cand[q][1] == t[1]) return q;
+    if (t[0] != cand[0][0] || t[1] < kMinWaveChunk) return -1;
+    *own = t[1];
+    return n;
+  };
+  int dep_own, pass_own;
+  const int ds = match(kDepCand, kNDep, tuning, &dep_own), ps = match(kPassCand, kNPass, tuning + 2, &pass_own);
   if (ds < 0 || ps < 0 || (tuning[4] != 0 && tuning[4] != 1))
     return set_error(ORBIT_ERR_ARG, "orbit_batch_set_tuning: not one of the candidate shapes");
   if (bt->used) ORBIT_CUDA(cudaStreamSynchronize(bt->stream));
+  if (dep_own != c.dep_own || pass_own != c.pass_own) bt->compiled = false;  // the block tables follow
+  c.dep_own = dep_own;
+  c.pass_own = pass_own;
   c.dep_sel = ds;
   c.pass_sel = ps;
   c.tune = ClassTuning{tuning[0], tuning[1], tuning[2], tuning[3], tuning[4]};

@@ -59,7 +59,7 @@ struct SolveJob {
 // Launch shapes of one class, chosen by the autotuner.
 struct ClassTuning {
   int dep_threads, dep_chunk;    // deposit: threads per block, particles per block
-  int pass_threads, pass_chunk;  // fused pass
+  int pass_threads, pass_chunk;  // fused pass (its FP64 form's threads; the fixed-point form has its own block size)
   int fft_wide;                  // 1: radix-2 stages, N/2 threads; 0: radix-4 stages, N/4 threads
 };
 
