@@ -13,19 +13,21 @@
 //
 // Accuracy.  The scales put the bunch's bound at 2^61 units at most: a rounding
 // is 2^-61 of the bound where binary64 rounds by 2^-53 of the value.  One scale
-// serves both planes and every particle, so it has to suit the smallest of x
-// and y (xp and yp) at its typical size, the geometric mean of the magnitudes
-// followed through the maps: the pass runs in fixed point only where each keeps
-// the 2^53 units of a double (fx::fine_enough).  Round beams have 2^55 to 2^58
-// of either, which is the room for planes apart.  Gaussian beams through random drifts, quadrupoles with fringes,
-// sextupoles and bends, planes up to a factor of 1e5 apart: the rms error of
-// each coordinate over binary64's on the same particles, by its typical size in
-// units: 2^55 0.45, 2^54 0.47 (at most 1.03), 2^53 0.57 (1.13), 2^52 0.68 (1.3),
-// 2^50 1.7 (3.6), 2^48 6.0.  The bound is the extent or 16 to 32 times the
-// geometric mean, whichever is less, so a few far particles cannot coarsen the
-// others' units; a particle beyond it, one whose kick exceeds a quarter of the
-// momentum bound, and one with |dp_p| >= 1/8 take the FP64 routines, and so does
-// the whole pass where the maps' constants do not fit the scales (prep_pass).
+// serves both planes and every particle, so it has to suit the smaller of x and
+// y (xp and yp) at its typical size, the geometric mean of a sample followed
+// through the maps: the pass runs in fixed point only where each keeps the 2^53
+// units of a double (fx::fine_enough).  Round beams have 2^55 to 2^58, which is
+// the room for planes apart.  Gaussian beams through random drifts, quadrupoles
+// with fringes, sextupoles and bends, planes up to a factor of 1e5 apart: rms
+// error of a coordinate over binary64's on the same particles, by its typical
+// size in units: 2^55 0.45, 2^54 0.47 (at most 1.03), 2^53 0.57 (1.13), 2^52 0.68
+// (1.3), 2^50 1.7 (3.6), 2^48 6.0.
+//
+// The bound is the extent or 16 to 32 times the geometric mean, whichever is
+// less, so a few far particles cannot coarsen the others' units; a particle
+// beyond it, one whose kick exceeds a quarter of the momentum bound, and one with
+// |dp_p| >= 1/8 take the FP64 routines, and so does the whole pass where the maps'
+// constants do not fit the scales (prep_pass).
 //
 // The functions are __host__ __device__: a host build checks them against
 // extended-precision maps.

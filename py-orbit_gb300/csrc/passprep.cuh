@@ -51,17 +51,36 @@ static __device__ __noinline__ void prep_pass(const PrepJob& J, const ScState* s
   float c[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) c[q] = lane <= nops ? o->f[q] : 0.f;
-  // typical magnitudes of x, xp, y, yp: the geometric mean of those that are not
-  // zero, which have to be half of the sample
-  unsigned cnt[4], most = 1u;
-  float mean[4];
-  for (int q = 0; q < 4; ++q) {
-    cnt[q] = (unsigned)(st->mag.exp[q] >> 32);
-    mean[q] = (float)(unsigned)st->mag.exp[q] / (float)max(cnt[q], 1u) - 60.f;
-    most = max(most, cnt[q]);
+  // typical magnitudes of x, xp, y, yp: the geometric mean, in whole exponents,
+  // of 256 particles spread over the bunch, of those that are not zero, which have
+  // to be half of them.  (Sampled by the pass in its loop they cost 1 to 2 us of
+  // every pass of 1e6 particles.)
+  unsigned sum[4] = {0u, 0u, 0u, 0u};  // exponents from 2^-60, and the count (2^20)
+  {
+    unsigned hw[8][4];  // high words, every load in flight at once
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int i = (int)(((long long)(r * 32 + lane) * J.n) >> 8);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) hw[r][q] = ok ? __ldcg(reinterpret_cast<const unsigned*>(J.c[q] + i) + 1) : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const unsigned e = hw[r][q] >> 20 & 0x7ffu;
+        if (e != 0u) sum[q] += (1u << 20) + min(max(e, 963u), 1083u) - 963u;
+      }
   }
-  for (int q = 0; q < 4; ++q) ok = ok && 2u * cnt[q] >= most;
-  fx::Typical ty = {exp2f(mean[0]), exp2f(mean[1]), exp2f(mean[2]), exp2f(mean[3])};
+  for (int q = 0; q < 4; ++q) sum[q] = __reduce_add_sync(0xffffffffu, sum[q]);
+  // (lane q of every four takes coordinate q)
+  const int lq = lane & 3;
+  const unsigned sq = lq == 0 ? sum[0] : lq == 1 ? sum[1] : lq == 2 ? sum[2] : sum[3], cnt = sq >> 20;
+  ok = ok && __reduce_min_sync(0xffffffffu, cnt) >= 128u;
+  const float mean_q = __fdividef((float)(sq & 0xfffffu), (float)max(cnt, 1u)) - 60.f, typ_q = exp2f(mean_q);
+  auto of = [](float v, int q) { return __shfl_sync(0xffffffffu, v, q); };
+  const float mean[4] = {of(mean_q, 0), of(mean_q, 1), of(mean_q, 2), of(mean_q, 3)};
+  fx::Typical ty = {of(typ_q, 0), of(typ_q, 1), of(typ_q, 2), of(typ_q, 3)};
   // bounds: the extent, or 16 to 32 times the larger plane's typical magnitude
   // where a few particles lie further out
   const int ex = (int)floorf(fmaxf(mean[0], mean[2])) + 5, ep = (int)floorf(fmaxf(mean[1], mean[3])) + 5;

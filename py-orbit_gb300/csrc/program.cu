@@ -88,29 +88,40 @@ struct FxFallback {
   const long long* Lm;
   double* c[5];
   const double* dE;
-  const double* knl;
+  double* knl;
   const KickArgs* kick;
   const MapCtx* m;
   const DevOp* ops;
   int a, b;
   unsigned long long mn[3], mx[3];
-  unsigned pm, ex[4];  // (ex: MagAcc::part sums)
+  unsigned pm;
   int bad;
   unsigned taken;  // particles the FP64 routines took
+  int fixed;       // the pass runs in fixed point
+  int declined;    // some of the block's particles are left to the FP64 routines
 };
 
 static_assert(kPassSmem + sizeof(FxFallback) + sizeof(PassPrep) + kCommitSmem + 64 <= kBlockSmem,
               "k_pass_fx: its own shared memory beside the largest copy of the potential");
 
+// A declined particle's 1/(1+dp_p) until the FP64 routines take it: minus
+// infinity, which the reciprocal of a sum never is.
+__device__ __forceinline__ double declined_mark() { return __hiloint2double((int)0xfff00000u, 0); }
+__device__ __forceinline__ bool declined(double knl) { return knl == declined_mark(); }
+
 // One particle by the FP64 routines: those the fixed-point form declines,
 // and all of a pass it cannot run.
 template <bool EXT>
-__device__ __noinline__ void pass_particle(FxFallback* f, int i, bool first) {
+__device__ __noinline__ void pass_particle(FxFallback* f, int i) {
   Part p;
   p.x = f->c[0][i]; p.xp = f->c[1][i]; p.y = f->c[2][i]; p.yp = f->c[3][i]; p.z = f->c[4][i]; p.dE = f->dE[i];
   p.knl = f->knl[i];
   p.dp_p = dmul<ORBIT_SOFT_MUL & 1>(p.dE, f->m->dp_p_coeff);
-  p.knl_ok = true;
+  p.knl_ok = !declined(p.knl);
+  if (!p.knl_ok) {  // the mark stands in its place
+    ensure_knl<ORBIT_SOFT_MUL & 1>(p, *f->m);
+    f->knl[i] = p.knl;
+  }
   if (!f->k->skip && bnd_inside(f->kick->bnd, p.x, p.y)) {
     if (!kick_fixed(*f->kf, f->P, f->Lm, p.x, p.y, p.z, p.xp, p.yp)) {
       kick_plain(*f->k, f->kick->phi, f->kick->lam, p.x, p.y, p.z, p.xp, p.yp);
@@ -131,12 +142,16 @@ __device__ __noinline__ void pass_particle(FxFallback* f, int i, bool first) {
     g.init();
     g.bound(p.xp, p.yp);
     atomicMax(&f->pm, g.pm);
-    if (first) {
-      g.sample(p.x, p.xp, p.y, p.yp);
-      for (int c = 0; c < 4; ++c) atomicAdd(&f->ex[c], g.part(c));
-    }
   }
   f->c[0][i] = p.x; f->c[1][i] = p.xp; f->c[2][i] = p.y; f->c[3][i] = p.yp; f->c[4][i] = p.z;
+}
+
+// Leaves particle i to the FP64 routines.  Out of line: with a call in its loop
+// the pass keeps its constants in shared memory (hoisted out of the loop they
+// spill) and its other registers as they are; marking in place was 1 to 3% slower.
+__device__ __noinline__ void fx_decline(FxFallback* f, int i) {
+  if (f->fixed) f->knl[i] = declined_mark();
+  f->declined = 1;
 }
 
 // Extrema of a pass run in fixed point: x and y as integers (their
@@ -260,7 +275,6 @@ __device__ __forceinline__ void pass_body(double* __restrict__ cx, double* __res
       if (sa.mag) {
         mag.bound(p.xp, p.yp);
         mag.em = max(mag.em, MagAcc::hi(p.dE));
-        if (i < nblk * (int)blockDim.x) mag.sample(p.x, p.xp, p.y, p.yp);
       }
     }
     if (km & KNL_STORE) {
@@ -280,7 +294,7 @@ __device__ __forceinline__ void pass_body(double* __restrict__ cx, double* __res
 // 1/(1+dp_p) unchanged, the plain form's kick.  A pass whose magnitudes or
 // constants do not fit (FxPass::ok, the same in every block) goes particle by
 // particle through the FP64 routines: 1e6 particles, 128 x 128 x 64, quadrupole
-// fringes beyond their limits, 324 us a kick (359 before the fixed-point form).
+// fringes beyond their limits, 328 us a kick (359 before the fixed-point form).
 //
 // Bound by the issue of integer instructions: 777 a particle for a kick and a
 // drift, about 1300 with two half quadrupoles and their fringes, at half an
@@ -298,7 +312,7 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
                                              double* __restrict__ cz, const double* __restrict__ cdE, int n,
                                              const DevOp* __restrict__ ops, int a, int b, const MapCtx& m,
                                              const KickArgs& kick, ScState* ext_st, unsigned* status,
-                                             const SetupArgs& sa, const double* __restrict__ knl_buf,
+                                             const SetupArgs& sa, double* __restrict__ knl_buf,
                                              const PassPrep* __restrict__ prep, int blk, int nblk) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ FxFallback s_f;
@@ -317,9 +331,11 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
       s_f.k = &s_prep.k; s_f.kf = &s_prep.kf;
       s_f.dE = cdE; s_f.knl = knl_buf; s_f.kick = &kick; s_f.m = &m; s_f.ops = ops; s_f.a = a; s_f.b = b;
       for (int c = 0; c < 3; ++c) { s_f.mn[c] = ~0ull; s_f.mx[c] = 0ull; }
-      s_f.pm = s_f.ex[0] = s_f.ex[1] = s_f.ex[2] = s_f.ex[3] = 0u;
+      s_f.pm = 0u;
       s_f.bad = 0;
       s_f.taken = 0u;
+      s_f.fixed = s_fx.ok;
+      s_f.declined = 0;
     }
   }
   if (KSMEM) fill_kick_grids<1>(kick, s_raw, blockDim.x > 64 ? 32 : 0);
@@ -327,6 +343,7 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
   const long long* P = KSMEM ? reinterpret_cast<const long long*>(s_raw) : kick.phi_fix;
   const long long* Lm = KSMEM ? P + (size_t)kick.nx * kick.ny : kick.lam_fix;
   const bool fixed = s_fx.ok != 0, bound = kick.bnd.type >= 0;
+  if (fixed && blk == 0 && threadIdx.x == 0) atomicAdd(&kick.st->n_fixed, 1ull);
   const fx::Scales s = s_fx.s;
   ExtFx ext;
   MagAcc mag;
@@ -334,62 +351,59 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
     ext.init();
     mag.init();
   }
-  // Particles left to the FP64 routines wait, for up to 31 rounds, as bits below
-  // a leading one, and a warp then takes them lane by lane together: it goes
-  // through those routines, 64 clocks an instruction, for any one of its lanes.
-  // Called at once, 5% of 1e6 particles declined made a kick 290 us (251 when
-  // every pass was of FP64), so 211.
   const int di = nblk * blockDim.x;
-  for (int i = first_particle(blk, nblk); i < n;) {
-    unsigned todo = 1u;
-    for (; !fixed && i < n && (int)todo > 0; i += di) todo += todo + 1u;
-    for (; fixed && i < n && (int)todo > 0; i += di) {
-      asm volatile("" ::: "memory");  // constants stay in shared memory: hoisted out of the loop they spill
-      fx::Part t;
-      const double x0 = cx[i], xp0 = cxp[i], y0 = cy[i], yp0 = cyp[i], dE = cdE[i];
+  for (int i = first_particle(blk, nblk); i < n; i += nblk * blockDim.x) {
+    bool ok = fixed;
+    fx::Part t;
+    if (ok) {
+      const double x = cx[i], xp = cxp[i], y = cy[i], yp = cyp[i], dE = cdE[i];
       const double knl = knl_buf[i];  // as an earlier pass of this run computed it from the same dE
       const double dp = __dmul_rn(dE, m.dp_p_coeff);
       t.z = cz[i];
-      t.x = fx::cvt_to(x0, s.x);
-      t.p = fx::cvt_to(xp0, s.p);
-      t.y = fx::cvt_to(y0, s.x);
-      t.r = fx::cvt_to(yp0, s.p);
-      bool ok = true;
+      t.x = fx::cvt_to(x, s.x);
+      t.p = fx::cvt_to(xp, s.p);
+      t.y = fx::cvt_to(y, s.x);
+      t.r = fx::cvt_to(yp, s.p);
       if (s_fx.check) {
         auto inside = [](double v, int lim) { return (__double2hiint(v) & 0x7fffffff) <= lim; };
-        ok = inside(x0, s_fx.limx) & inside(y0, s_fx.limx) & inside(xp0, s_fx.limp) & inside(yp0, s_fx.limp) &
+        ok = inside(x, s_fx.limx) & inside(y, s_fx.limx) & inside(xp, s_fx.limp) & inside(yp, s_fx.limp) &
              inside(dp, s_fx.limd);
       }
-      if (ok && (!bound || bnd_inside(kick.bnd, x0, y0))) {
+      if (ok && (!bound || bnd_inside(kick.bnd, x, y))) {
         ok = kick_fx(s_fx, kick.nx, P, Lm, t);
       }
-      todo += todo;
-      if (!ok) {
-        ++todo;
-        continue;
-      }
       fx::part_init(t, fx::kappa_of(knl), fx::cvt_to(dp, s.k), s.k);
-      fx::apply(t, s_fx.op, s_fx.n, s);
-      const double x = fx::cvt_from(t.x, s.x), xp = fx::cvt_from(t.p, s.p), y = fx::cvt_from(t.y, s.x), yp = fx::cvt_from(t.r, s.p);
-      const double z = t.z + fx::cvt_from(t.d, s.d);
-      if (EXT) {
-        ext.add(t.x, t.y, z);
-        mag.bound(xp, yp);
-        if (i < di) mag.sample(x, xp, y, yp);  // the thread's first particle
-      }
-      cx[i] = x; cxp[i] = xp; cy[i] = y; cyp[i] = yp; cz[i] = z;
     }
-    todo ^= 1u << (31 - __clz(todo));
-    if (todo) atomicAdd(&s_f.taken, (unsigned)__popc(todo));
-    for (; todo; todo &= todo - 1u) {
-      const int q = i - __ffs(todo) * di;
-      pass_particle<EXT>(&s_f, q, q < di);
+    if (!ok) {
+      fx_decline(&s_f, i);
+      continue;
     }
+    fx::apply(t, s_fx.op, s_fx.n, s);
+    const double x = fx::cvt_from(t.x, s.x), xp = fx::cvt_from(t.p, s.p), y = fx::cvt_from(t.y, s.x), yp = fx::cvt_from(t.r, s.p);
+    const double z = t.z + fx::cvt_from(t.d, s.d);
+    if (EXT) {
+      ext.add(t.x, t.y, z);
+      mag.bound(xp, yp);
+    }
+    cx[i] = x; cxp[i] = xp; cy[i] = y; cyp[i] = yp; cz[i] = z;
   }
-  __syncthreads();  // the fallback's shared extrema and count
-  if (threadIdx.x == 0) {
-    if (blk == 0 && fixed) kick.st->n_fixed += 1;
-    if (s_f.taken) atomicAdd(&kick.st->n_fp64, (unsigned long long)s_f.taken);
+  __syncthreads();
+  // A warp goes through the FP64 routines, 64 clocks an instruction, for any one
+  // of its lanes: the declined particles wait for the end of the loop, and every
+  // 32 rounds' are then taken lane by lane together.  Taken at once, 5% of 1e6
+  // particles far out made a kick 290 us (251 when every pass was of FP64), so
+  // 215.
+  if (s_f.declined) {
+    for (int i = first_particle(blk, nblk); i < n;) {
+      unsigned todo = 0u;
+      const int i0 = i;
+      for (int r = 0; r < 32 && i < n; ++r, i += di)
+        if (!fixed || declined(knl_buf[i])) todo |= 1u << r;
+      if (todo) atomicAdd(&s_f.taken, (unsigned)__popc(todo));
+      for (; todo; todo &= todo - 1u) pass_particle<EXT>(&s_f, i0 + (__ffs(todo) - 1) * di);
+    }
+    __syncthreads();  // their extrema and count
+    if (threadIdx.x == 0) atomicAdd(&kick.st->n_fp64, (unsigned long long)s_f.taken);
   }
   // the last block sets up the grids of the next kick
   if (EXT) {
@@ -406,7 +420,7 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
       // dE is unchanged; without magnitudes before, none are claimed
       mag.em = kick.st->mag.pmax ? kick.st->mag.emax : 0x7fefffffu;
     }
-    if (sa.mag) mag_block_commit(mag, ext_st, s_f.ex);
+    if (sa.mag) mag_block_commit(mag, ext_st);
     ext_commit_and_setup(acc, ext_st, status, sa, nblk);
   }
 }
@@ -431,7 +445,7 @@ __global__ void __launch_bounds__(ORBIT_FX_THREADS) k_pass_fx(double* __restrict
                                               const __grid_constant__ MapCtx m,
                                               const __grid_constant__ KickArgs kick, ScState* ext_st,
                                               unsigned* status, const __grid_constant__ SetupArgs sa,
-                                              const double* __restrict__ knl_buf,
+                                              double* __restrict__ knl_buf,
                                               const PassPrep* __restrict__ prep) {
   pass_fx_body<EXT, KSMEM>(cx, cxp, cy, cyp, cz, cdE, n, ops, a, b, m, kick, ext_st, status, sa, knl_buf,
                                prep, blockIdx.x, gridDim.x);
@@ -766,6 +780,8 @@ static int enqueue_turn(orbit_program_t* p, orbit_bunch_t* bu, cudaStream_t s, c
     std::memset(&job, 0, sizeof(job));
     if (fixed_pass(sg, kc->form == ORBIT_FORM_PLAIN && !kc->rb, km)) {
       job.ops = ops; job.a = sg.a; job.b = sg.b;
+      for (int q = 0; q < 4; ++q) job.c[q] = bu->coord(q);
+      job.n = bu->n;
       job.dp_p_coeff = m.dp_p_coeff;
       job.host_factor = sc_host_factor(bu->sync, len_of(i));
       job.out = kc->d_prep;

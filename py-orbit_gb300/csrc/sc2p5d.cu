@@ -1099,6 +1099,8 @@ __global__ void kb_rows_fwd(const SolveJob* __restrict__ jobs, FftPlan pl, int n
     if (pass) {
       const PassJob& Q = pass[blockIdx.y];
       prep.ops = Q.ops; prep.a = a; prep.b = b;
+      for (int k = 0; k < 4; ++k) prep.c[k] = Q.c[k];
+      prep.n = Q.n;
       prep.dp_p_coeff = Q.m.dp_p_coeff;
       prep.host_factor = Q.ka.host_factor;
       prep.out = Q.prep;

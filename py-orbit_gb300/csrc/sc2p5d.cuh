@@ -44,15 +44,11 @@ struct ScState {
   unsigned conv_bar[2];
   // magnitudes of the bunch for the fixed-point maps of the next pass,
   // accumulated by a lattice pass beside the extrema: largest high words of
-  // |xp|, |yp| and of |dE|; of x, xp, y, yp the sums of the exponents (clamped
-  // to 2^-60..2^60, from 0) over one particle of every thread, with the number
-  // of those that are not zero above them (2^32); the set-up moves them to `mag`
-  // (zero after a scan that has none)
+  // |xp|, |yp| and of |dE|; the set-up moves them to `mag` (zero after a scan that
+  // has none)
   unsigned acc_pmax, acc_emax;
-  unsigned long long acc_exp[4];
   struct {
     unsigned pmax, emax;
-    unsigned long long exp[4];
     double xmax;  // max |x|, |y| before the grid is stretched
   } mag;
 };
@@ -115,11 +111,13 @@ struct DevOp;
 struct PassPrep;
 struct LogTab;
 // The lattice pass that follows a kick, for the constants made beside its
-// solve (prep_pass): maps ops[a..b), dp_p per dE and the kick factor; out
-// null: none.
+// solve (prep_pass): maps ops[a..b), dp_p per dE, the kick factor and the
+// bunch's x, xp, y, yp; out null: none.
 struct PrepJob {
   const DevOp* ops;
   int a, b;
+  const double* c[4];
+  int n;
   double dp_p_coeff, host_factor;
   PassPrep* out;
 };

@@ -37,59 +37,37 @@ struct ExtAcc {
   }
 };
 
-// Magnitudes of a bunch (ScState::mag): largest high words of |xp|, |yp| and
-// |dE|, and the clamped exponents of x, xp, y, yp of one particle a thread, a
-// byte each: 0 for zero, else 128 + the exponent from 2^-60.
+// Magnitudes of a bunch (ScState::mag): largest high words of |xp|, |yp| and of
+// |dE|.
 struct MagAcc {
-  unsigned pm, em, ex;
-  __device__ __forceinline__ void init() { pm = em = ex = 0u; }
+  unsigned pm, em;
+  __device__ __forceinline__ void init() { pm = em = 0u; }
   static __device__ __forceinline__ unsigned hi(double v) {
     return (unsigned)__double2hiint(v) & 0x7fffffffu;
   }
-  static __device__ __forceinline__ unsigned ex_of(double v) {
-    const unsigned h = hi(v) >> 20;
-    return h == 0u ? 0u : min(max(h, 963u), 1083u) - 835u;
-  }
   __device__ __forceinline__ void bound(double xp, double yp) { pm = max(pm, max(hi(xp), hi(yp))); }
-  __device__ __forceinline__ void sample(double x, double xp, double y, double yp) {
-    ex = ex_of(x) | ex_of(xp) << 8 | ex_of(y) << 16 | ex_of(yp) << 24;
-  }
-  // Coordinate c's byte as exponent and, above it (2^20), the count.
-  __device__ __forceinline__ unsigned part(int c) const {
-    const unsigned b = ex >> (8 * c) & 255u;
-    return (b & 127u) | (b >> 7) << 20;
-  }
 };
 
-// Block-wide reduction, one atomic per quantity per block; more: part() sums of
-// other particles of the block, in shared memory.  Integer maxima and sums: the
-// same on every run.
-__device__ __forceinline__ void mag_block_commit(const MagAcc& a, ScState* st, const unsigned* more = nullptr) {
-  __shared__ unsigned s_m[6][32];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned full = 0xffffffffu;
-  const unsigned v[6] = {__reduce_max_sync(full, a.pm),      __reduce_max_sync(full, a.em),
-                         __reduce_add_sync(full, a.part(0)), __reduce_add_sync(full, a.part(1)),
-                         __reduce_add_sync(full, a.part(2)), __reduce_add_sync(full, a.part(3))};
-  if (lane == 0)
-    for (int k = 0; k < 6; ++k) s_m[k][w] = v[k];
+// Block-wide reduction, one atomic per quantity per block.
+__device__ __forceinline__ void mag_block_commit(const MagAcc& a, ScState* st) {
+  __shared__ unsigned s_m[2][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+  const unsigned full = 0xffffffffu, pm = __reduce_max_sync(full, a.pm), em = __reduce_max_sync(full, a.em);
+  if (lane == 0) {
+    s_m[0][w] = pm;
+    s_m[1][w] = em;
+  }
   __syncthreads();
-  if (w < 6) {  // one warp per quantity (a block has at least that many, or its warps take turns)
-    const int nw = (blockDim.x + 31) >> 5;
-    for (int k = w; k < 6; k += nw) {
-      const unsigned u = lane < nw ? s_m[k][lane] : 0u;
-      unsigned r = k < 2 ? __reduce_max_sync(full, u) : __reduce_add_sync(full, u);
-      if (lane == 0) {
-        if (k >= 2 && more) r += more[k - 2];
-        if (k < 2) atomicMax(k == 0 ? &st->acc_pmax : &st->acc_emax, r);
-        else atomicAdd(&st->acc_exp[k - 2], ((unsigned long long)(r >> 20) << 32) | (r & 0xfffffu));
-      }
-    }
+  if (w == 0) {
+    const unsigned r0 = __reduce_max_sync(full, lane < nw ? s_m[0][lane] : 0u);
+    const unsigned r1 = __reduce_max_sync(full, lane < nw ? s_m[1][lane] : 0u);
+    if (lane == 0) atomicMax(&st->acc_pmax, r0);
+    if (lane == 1) atomicMax(&st->acc_emax, r1);
   }
 }
 
 // Static shared memory of mag_block_commit, ext_block_commit and last_block_done.
-static const size_t kCommitSmem = 6 * 32 * (sizeof(unsigned) + sizeof(unsigned long long)) + 16;
+static const size_t kCommitSmem = 32 * (2 * sizeof(unsigned) + 6 * sizeof(unsigned long long)) + 16;
 
 // Smallest 64-bit key of a warp, from two 32-bit reductions.
 __device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
@@ -150,8 +128,6 @@ static __device__ __noinline__ void sc_setup_warp(ScState* st, unsigned* status,
   const unsigned stat = __ldcg(status);
   // every load before the first store: one trip to L2, not one each
   const unsigned pmax = __ldcg(&st->acc_pmax), emax = __ldcg(&st->acc_emax);
-  const unsigned long long mexp[4] = {__ldcg(&st->acc_exp[0]), __ldcg(&st->acc_exp[1]), __ldcg(&st->acc_exp[2]),
-                                      __ldcg(&st->acc_exp[3])};
   const int dirty = st->green_dirty;
   double xMin = dkey_inv(key[0]), xMax = dkey_inv(key[1]);
   double yMin = dkey_inv(key[2]), yMax = dkey_inv(key[3]);
@@ -161,10 +137,8 @@ static __device__ __noinline__ void sc_setup_warp(ScState* st, unsigned* status,
     for (int c = 0; c < 3; ++c) { st->key[2 * c] = ~0ull; st->key[2 * c + 1] = 0ull; }
     st->mag.pmax = pmax;
     st->mag.emax = emax;
-    for (int c = 0; c < 4; ++c) st->mag.exp[c] = mexp[c];
     st->mag.xmax = fmax(fmax(fabs(xMin), fabs(xMax)), fmax(fabs(yMin), fabs(yMax)));
     st->acc_pmax = st->acc_emax = 0u;
-    for (int c = 0; c < 4; ++c) st->acc_exp[c] = 0ull;
     st->conv_bar[0] = 0u;
     st->conv_bar[1] = 0u;
   }

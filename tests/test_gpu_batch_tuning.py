@@ -41,6 +41,34 @@ def test_shapes_of_other_bunches(shape, grid):
         assert np.array_equal(a.getCoordinates(), b.getCoordinates())
 
 
+def test_shapes_change_no_bit_of_beams_at_the_limits_of_fixed_point():
+    """Flat beams and beams with a halo: whether a pass runs in fixed point, and
+    in which units, hangs on the bunch alone."""
+    from orbit_gb300 import workloads as W
+    from orbit_gb300.batch import BunchBatch
+    from spacecharge import SpaceChargeCalc2p5D
+
+    def run(shape):
+        members = []
+        for k in range(24):
+            c = W.c2_coords(3001 + 997 * k, seed=k)
+            c[2:4] *= 0.03 * 1.1 ** k
+            if k % 3 == 0:
+                c[:4, :: 17 + k] *= 60.0
+            members.append((W.make_bunch(np.ascontiguousarray(c), 1e6),
+                            W.fodo_lattice(SpaceChargeCalc2p5D(32, 32, 8), cells=1)))
+        batch = BunchBatch(members)
+        batch.classes()
+        batch._batch.set_tuning(0, *shape)
+        batch.trackTurns(2)
+        return [b.getCoordinates() for b, _ in members]
+
+    want = run((768, 8192, 512, 4096, 1))
+    for shape in ((768, 2632, 512, 256, 1), (512, 8192, 512, 16384, 1)):
+        for k, (a, b) in enumerate(zip(run(shape), want)):
+            assert np.array_equal(a, b), k
+
+
 @pytest.mark.parametrize("shape", [(768, 255, 512, 4096, 1), (640, 8192, 512, 4096, 1), (768, 8192, 640, 4096, 1),
                                    (768, 8192, 512, -1, 1), (768, 8192, 512, 4096, 2)])
 def test_other_shapes_are_refused(shape):
