@@ -23,11 +23,11 @@
 // size in units: 2^55 0.45, 2^54 0.47 (at most 1.03), 2^53 0.57 (1.13), 2^52 0.68
 // (1.3), 2^50 1.7 (3.6), 2^48 6.0.
 //
-// The bound is the extent or 16 to 32 times the geometric mean, whichever is
-// less, so a few far particles cannot coarsen the others' units; a particle
-// beyond it, one whose kick exceeds a quarter of the momentum bound, and one with
-// |dp_p| >= 1/8 take the FP64 routines, and so does the whole pass where the maps'
-// constants do not fit the scales (prep_pass).
+// The bound is the extent or 24 times the typical size, whichever is less, so a
+// few far particles cannot coarsen the others' units; a particle beyond it, one
+// whose kick exceeds a quarter of the momentum bound, and one with |dp_p| >= 1/8
+// take the FP64 routines, and so does the whole pass where the maps' constants do
+// not fit the scales (prep_pass).
 //
 // The functions are __host__ __device__: a host build checks them against
 // extended-precision maps.

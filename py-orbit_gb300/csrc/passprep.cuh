@@ -18,7 +18,8 @@ struct FxGrid {      // t = x / step - min / step in units of 2^-F
   int F, lo, hi, half;  // high words: a quarter cell inside the edges, 1/2
 };
 struct alignas(16) FxPass {
-  int ok;             // the pass runs in fixed point
+  int ok;             // the pass runs in fixed point: its scales and maps fit
+  int kick_ok;        // and so do the kick's constants
   int n;              // maps
   int check;          // some particles lie beyond the bounds
   fx::Scales s;
@@ -38,10 +39,9 @@ struct alignas(16) PassPrep {
   FxPass fx;
 };
 
-// Executed by one warp.  What hangs on the line density (the kick's factor) is
-// made last: with `bar`, after n blocks have arrived there.
-static __device__ __noinline__ void prep_pass(const PrepJob& J, const ScState* st, int nx, int ny, int nz,
-                                              unsigned* bar, unsigned nblk, long long polls, unsigned* status) {
+// The scales, the maps' constants and the grids' (one warp): nothing here hangs
+// on the solve.
+__device__ __forceinline__ void prep_maps(const PrepJob& J, const ScState* st, int nx, int ny, int nz) {
   const int lane = threadIdx.x & 31, nops = J.b - J.a;
   FxPass* f = &J.out->fx;
   // lane 0 the segment's start entry, lanes 1..nops its maps
@@ -77,17 +77,18 @@ static __device__ __noinline__ void prep_pass(const PrepJob& J, const ScState* s
   const int lq = lane & 3;
   const unsigned sq = lq == 0 ? sum[0] : lq == 1 ? sum[1] : lq == 2 ? sum[2] : sum[3], cnt = sq >> 20;
   ok = ok && __reduce_min_sync(0xffffffffu, cnt) >= 128u;
-  const float mean_q = __fdividef((float)(sq & 0xfffffu), (float)max(cnt, 1u)) - 60.f, typ_q = exp2f(mean_q);
+  const float typ_q = exp2f(__fdividef((float)(sq & 0xfffffu), (float)max(cnt, 1u)) - 60.f);
   auto of = [](float v, int q) { return __shfl_sync(0xffffffffu, v, q); };
-  const float mean[4] = {of(mean_q, 0), of(mean_q, 1), of(mean_q, 2), of(mean_q, 3)};
   fx::Typical ty = {of(typ_q, 0), of(typ_q, 1), of(typ_q, 2), of(typ_q, 3)};
-  // bounds: the extent, or 16 to 32 times the larger plane's typical magnitude
-  // where a few particles lie further out
-  const int ex = (int)floorf(fmaxf(mean[0], mean[2])) + 5, ep = (int)floorf(fmaxf(mean[1], mean[3])) + 5;
+  // bounds: the extent, or 24 times the larger plane's typical size (9 standard
+  // deviations of a Gaussian) where a few particles lie further out.  16 made a
+  // batch of tracked bunches, whose tails it cut, 1% slower, since one particle's
+  // way through the FP64 routines takes 15 us; 50 leaves a beam with a halo too few
+  // units
   const float xm = (float)st->mag.xmax * 1.0001f;
   const float pm = (float)__hiloint2double((int)st->mag.pmax, -1) * 1.0001f;
   const float dm = (float)__hiloint2double((int)st->mag.emax, -1) * fabsf((float)J.dp_p_coeff) * 1.0001f;
-  const float x0 = fminf(xm, ldexpf(1.f, ex)), p0 = fminf(pm, ldexpf(1.f, ep)), d0 = fminf(dm, 0.124f);
+  const float x0 = fminf(xm, 24.f * fmaxf(ty.x, ty.y)), p0 = fminf(pm, 24.f * fmaxf(ty.p, ty.r)), d0 = fminf(dm, 0.124f);
   fx::Bounds bd = {x0, 1.25f * p0, d0, 0.f, 0.f, 0};
   if (ok) {
     for (int q = 1; q <= nops; ++q) {
@@ -159,27 +160,42 @@ static __device__ __noinline__ void prep_pass(const PrepJob& J, const ScState* s
       f->Fz = 57 - width(nz);
     }
   }
+  if (lane == 0) f->ok = ok ? 1 : 0;
+}
+
+// The kick's constants (one thread), which hang on the finished line density.
+__device__ __forceinline__ void prep_kick(const PrepJob& J, const ScState* st, int nx, int ny, int nz) {
+  FxPass* f = &J.out->fx;
+  KickConst kc;
+  KickFix kx;
+  load_kick_const(kc, st, J.host_factor, nx, ny, nz, false);
+  J.out->k = kc;
+  load_kick_fix(kx, st, kc.fac, nx, ny, nz);
+  J.out->kf = kx;
+  const double gx = -kc.fac * kx.ax, gy = -kc.fac * kx.ay;
+  const int e = max(fx::exp_of(gx), fx::exp_of(gy));
+  f->ce = e;
+  bool ok = true;
+  if (e < -2000) {  // no kick
+    f->Cx = f->Cy = fx::V{0, 0};
+  } else {
+    ok = fx::fixv(gx, 61 - e, &f->Cx) && fx::fixv(gy, 61 - e, &f->Cy);
+  }
+  f->kick_ok = ok ? 1 : 0;
+}
+
+// Executed by one warp: `maps`, then `kick`, the latter with `bar` after nblk
+// blocks have arrived there.  The fused convolution gives both to one block; the
+// separate forward rows give them to two, which run side by side.
+static __device__ __noinline__ void prep_pass(const PrepJob& J, const ScState* st, int nx, int ny, int nz, bool maps,
+                                              bool kick, unsigned* bar, unsigned nblk, long long polls,
+                                              unsigned* status) {
+  if (maps) prep_maps(J, st, nx, ny, nz);
   if (bar) {
-    if (lane == 0) counter_wait(bar, nblk, polls, status);
+    if ((threadIdx.x & 31) == 0) counter_wait(bar, nblk, polls, status);
     __syncwarp();
   }
-  if (lane == 0) {
-    KickConst kc;
-    KickFix kx;
-    load_kick_const(kc, st, J.host_factor, nx, ny, nz, false);
-    J.out->k = kc;
-    load_kick_fix(kx, st, kc.fac, nx, ny, nz);
-    J.out->kf = kx;
-    const double gx = -kc.fac * kx.ax, gy = -kc.fac * kx.ay;
-    const int e = max(fx::exp_of(gx), fx::exp_of(gy));
-    f->ce = e;
-    if (e < -2000) {  // no kick
-      f->Cx = f->Cy = fx::V{0, 0};
-    } else if (!fx::fixv(gx, 61 - e, &f->Cx) || !fx::fixv(gy, 61 - e, &f->Cy)) {
-      ok = false;
-    }
-    f->ok = ok ? 1 : 0;
-  }
+  if (kick && (threadIdx.x & 31) == 0) prep_kick(J, st, nx, ny, nz);
 }
 
 // Executed by warp 0 of a block: the constants (with those of nops maps) into
@@ -221,7 +237,7 @@ __device__ __forceinline__ void load_prep(const PassPrep* __restrict__ prep, con
       j = 0;
     }
     f->j = j;
-    if (j > 29) f->ok = 0;
+    if (j > 29 || !f->kick_ok) f->ok = 0;
     else f->limj = 1 << (29 - j);
   }
 }

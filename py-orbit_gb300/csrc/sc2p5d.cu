@@ -221,11 +221,15 @@ __device__ __forceinline__ void rows_fwd_body(ScState* st, void* src, double* rh
   typedef typename CT<T>::t C;
   if (SRC == 0 && gate && !st->green_dirty) return;
   if (st->skip) return;
+  if (SRC == 1 && blk == nblk) {  // an extra block, of launches with a pass to prepare
+    if (threadIdx.x < 32) prep_pass(*prep, st, nrows, ncols, nz, true, false, nullptr, 0, 0, nullptr);
+    return;
+  }
   if (SRC == 1 && blk == nblk - 1) {
     finalize_block(st, (unsigned long long*)zacc, nz, lam, lam_f, reset_dirty);
     if (prep && prep->out) {
       __syncthreads();
-      if (threadIdx.x < 32) prep_pass(*prep, st, nrows, ncols, nz, nullptr, 0, 0, nullptr);
+      if (threadIdx.x < 32) prep_pass(*prep, st, nrows, ncols, nz, false, true, nullptr, 0, 0, nullptr);
     }
     return;
   }
@@ -314,7 +318,7 @@ __global__ void k_rows_fwd(ScState* st, void* src, double* rho_out, typename CT<
                            int gate, void* zacc, int nz, double* lam, float* lam_f,
                            const __grid_constant__ PrepJob prep) {
   rows_fwd_body<T, SRC>(st, src, rho_out, hat, tw, pl, nrows, ncols, H, gate, zacc, nz, lam, lam_f, blockIdx.x,
-                        gridDim.x, nullptr, nullptr, true, &prep);
+                        gridDim.x - (prep.out ? 1 : 0), nullptr, nullptr, true, &prep);
 }
 
 // Column transforms along x (length N = nx2), one column k per block.
@@ -540,7 +544,7 @@ __global__ void k_conv_fused(const __grid_constant__ ConvArgs A) {
         atomicAdd(&st->conv_bar[0], 1u);
         atomicAdd(&st->conv_bar[1], 1u);
       }
-      prep_pass(A.prep, st, A.nx, A.ny, A.nz, &st->conv_bar[0], gridDim.x, A.wait_polls, A.status);
+      prep_pass(A.prep, st, A.nx, A.ny, A.nz, true, true, &st->conv_bar[0], gridDim.x, A.wait_polls, A.status);
     }
     return;
   }
@@ -1106,7 +1110,7 @@ __global__ void kb_rows_fwd(const SolveJob* __restrict__ jobs, FftPlan pl, int n
       prep.out = Q.prep;
     }
     rows_fwd_body<double, 1>(J.st, J.rho_q, J.rho, J.hat, J.tw_y, pl, nrows, ncols, H, 1, J.z_q, nz, J.lam, nullptr,
-                             blockIdx.x, gridDim.x, nullptr, nullptr, true, &prep);
+                             blockIdx.x, gridDim.x - (pass ? 1 : 0), nullptr, nullptr, true, &prep);
   }
 }
 
@@ -1372,7 +1376,7 @@ static int enqueue_rows_fwd(orbit_sc2p5d_t* c, cudaStream_t s, const PrepJob& pr
   const C* twy = (const C*)c->d_tw_y;
   int thy = fft_threads(c->plan_y);
   size_t smy = fft_smem<T>(c->ny2);
-  int blocks = (c->nx + 1) / 2 + 1;
+  int blocks = (c->nx + 1) / 2 + 1 + (prep.out ? 1 : 0);
   ORBIT_PB("fft_rows_fwd", s);
   k_rows_fwd<T, 1><<<blocks, thy, smy, s>>>(c->d_st, c->d_rho_q, c->d_rho, hat, twy, c->plan_y, c->nx, c->ny,
                                             c->H, 1, c->d_z_q, c->nz, c->d_lam, c->d_lam_f, prep);
@@ -1536,7 +1540,7 @@ int batch_enqueue_solve(const SolveJob* jobs, int nm, const orbit_sc2p5d_t* c, i
   int thx = batch_fft_threads(c->plan_x, fft_wide), thy = batch_fft_threads(c->plan_y, fft_wide);
   size_t smx = fft_smem<double>(c->nx2), smy = fft_smem<double>(c->ny2);
   ORBIT_PB("batch_rows_fwd", s);
-  kb_rows_fwd<1><<<dim3((c->nx + 1) / 2 + 1, nm), thy, smy, s>>>(jobs, c->plan_y, c->nx, c->ny, c->H, c->nz,
+  kb_rows_fwd<1><<<dim3((c->nx + 1) / 2 + 1 + (pass ? 1 : 0), nm), thy, smy, s>>>(jobs, c->plan_y, c->nx, c->ny, c->H, c->nz,
                                                                      pass, a, b);
   ORBIT_PE(s);
   ORBIT_PB("batch_cols_conv", s);
