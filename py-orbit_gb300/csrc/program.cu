@@ -294,7 +294,7 @@ __device__ __forceinline__ void pass_body(double* __restrict__ cx, double* __res
 // 1/(1+dp_p) unchanged, the plain form's kick.  A pass whose magnitudes or
 // constants do not fit (FxPass::ok, the same in every block) goes particle by
 // particle through the FP64 routines: 1e6 particles, 128 x 128 x 64, quadrupole
-// fringes beyond their limits, 328 us a kick (359 before the fixed-point form).
+// fringes beyond their limits, 327 us a kick (359 before the fixed-point form).
 //
 // Bound by the issue of integer instructions: 777 a particle for a kick and a
 // drift, about 1300 with two half quadrupoles and their fringes, at half an
@@ -392,7 +392,7 @@ __device__ __forceinline__ void pass_fx_body(double* __restrict__ cx, double* __
   // of its lanes: the declined particles wait for the end of the loop, and every
   // 32 rounds' are then taken lane by lane together.  Taken at once, 5% of 1e6
   // particles far out made a kick 290 us (251 when every pass was of FP64), so
-  // 215.
+  // 216.
   if (s_f.declined) {
     for (int i = first_particle(blk, nblk); i < n;) {
       unsigned todo = 0u;

@@ -1,6 +1,7 @@
 """Which lattice passes run in fixed point and how many particles their FP64
 routines take (SpaceChargeCalc2p5D's pass_counters), with the coordinates
-against the oracle: a declined particle waits up to 31 rounds of its thread.
+against the oracle: declined particles wait for the end of the block's loop and
+are taken 32 rounds of a thread at a time.
 
 Tolerance: as tests/test_gpu_fixed_pass.py, 2e-11 over at most 20 kicks."""
 import numpy as np
@@ -32,7 +33,7 @@ def _coords(n, kind):
     (20_000, "plain", "strong", (32, 32, 8), 0.0, 1.0, 1.0),
     (100_003, "halo", "drifts", (64, 64, 16), 1.0, 0.9 * HALO, 1.1 * HALO),
     (33_333, "halo", "fodo", (256, 256, 4), 1.0, 0.9 * HALO, 1.1 * HALO),
-    (3_300_000, "halo", "drifts", (128, 128, 4), 1.0, 0.9 * HALO, 1.1 * HALO),  # more than 31 rounds a thread
+    (3_300_000, "halo", "drifts", (128, 128, 4), 1.0, 0.9 * HALO, 1.1 * HALO),  # more than 32 rounds a thread
 ])
 def test_fixed_passes_and_their_exceptions(n, beam, lattice, grid, fixed, low, high):
     from spacecharge import SpaceChargeCalc2p5D
